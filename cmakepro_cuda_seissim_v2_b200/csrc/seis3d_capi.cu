@@ -287,6 +287,7 @@ struct seis3d_session {
         const float weights[4] = {SEIS3D_W0, SEIS3D_W1, SEIS3D_W2, SEIS3D_W3};
         for (int r = 0; r < 4; ++r) G.w[r] = weights[r];
         G.w[4] = G.invH;
+        for (int r = 0; r < 5; ++r) G.w2[r] = make_float2(G.w[r], G.w[r]);
         G.h = ctx.spacing3D;
         G.dt = ctx.dt3D;
         G.frequency = ctx.frequency3D;
@@ -639,30 +640,31 @@ namespace {
 void buildTensorMaps(seis3d_session* s) {
     const EncodeTiled encode = encoder();
     std::vector<CUtensorMap> table(tma::kMapCount);
-    const cuuint64_t dims[3] = {cuuint64_t(s->ctx.gx3D), cuuint64_t(s->ctx.gy3D), cuuint64_t(s->ctx.gz3D)};
-    const cuuint64_t strides[2] = {cuuint64_t(s->pitch) * 4, cuuint64_t(s->plane) * 4};
-    const cuuint32_t unit[3] = {1, 1, 1};
-    auto make = [&](int index, float* base, cuuint32_t w, cuuint32_t h) {
-        const cuuint32_t box[3] = {w, h, 1};
-        const CUresult r = encode(&table[index], CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 3, base, dims, strides, box, unit,
+    // `count` volumes from `base`, `apart` volumes from one to the next; boxes `planes` deep.
+    auto make = [&](int index, float* base, int count, int apart, cuuint32_t w, cuuint32_t h, cuuint32_t planes = 1) {
+        const cuuint64_t dims[4] = {cuuint64_t(s->ctx.gx3D), cuuint64_t(s->ctx.gy3D), cuuint64_t(s->ctx.gz3D), cuuint64_t(count)};
+        const cuuint64_t volume = cuuint64_t(s->plane) * cuuint64_t(s->ctx.gz3D);
+        const cuuint64_t strides[3] = {cuuint64_t(s->pitch) * 4, cuuint64_t(s->plane) * 4, volume * 4 * cuuint64_t(apart)};
+        const cuuint32_t unit[4] = {1, 1, 1, 1};
+        const cuuint32_t box[4] = {w, h, planes, cuuint32_t(count)};
+        const CUresult r = encode(&table[index], CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 4, base, dims, strides, box, unit,
                                   CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE,
                                   CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
         if (r != CUDA_SUCCESS) throw RuntimeError("Seis3D: cuTensorMapEncodeTiled failed (" + std::to_string(int(r)) + ").");
     };
-    for (int k = 0; k < 9; ++k) make(tma::kCenter0 + k, s->field[k], kTX, kTY);
-    make(tma::kCenter0 + 9, s->invRho, kTX, kTY);
-    make(tma::kCenter0 + 10, s->lambda, kTX, kTY);
-    make(tma::kCenter0 + 11, s->mu, kTX, kTY);
-    make(tma::kSxxX, s->field[3], kTX + 8, kTY);
-    make(tma::kSxzX, s->field[8], kTX + 8, kTY);
-    make(tma::kSxyXY, s->field[6], kTX + 8, kTY + 8);
-    make(tma::kSyyY, s->field[4], kTX, kTY + 8);
-    make(tma::kSyzY, s->field[7], kTX, kTY + 8);
-    make(tma::kVxXY, s->field[0], kTX + 8, kTY + 8);
-    make(tma::kVyXY, s->field[1], kTX + 8, kTY + 8);
-    make(tma::kVzXY, s->field[2], kTX + 8, kTY + 8);
-    make(tma::kRhoT, s->invRho, 36, kTY + 1);
-    make(tma::kMuT, s->mu, 36, kTY + 1);
+    make(tma::kSxxSxz, s->field[3], 2, 5, kTX + 8, kTY);
+    make(tma::kSxy, s->field[6], 1, 1, kTX + 8, kTY + 8);
+    make(tma::kSyySyz, s->field[4], 2, 3, kTX, kTY + 8);
+    make(tma::kRhoTwo, s->invRho, 1, 1, 36, kTY + 1, 2);
+    make(tma::kVelocity, s->field[0], 3, 1, kTX, kTY);
+    make(tma::kSyzSxzCentre, s->field[7], 2, 1, kTX, kTY);
+    make(tma::kSzzCentre, s->field[5], 1, 1, kTX, kTY);
+    make(tma::kVelocityHalo, s->field[0], 3, 1, kTX + 8, kTY + 8);
+    make(tma::kMuTwo, s->mu, 1, 1, 36, kTY + 1, 2);
+    make(tma::kLambda, s->lambda, 1, 1, kTX, kTY);
+    make(tma::kStress, s->field[3], 6, 1, kTX, kTY);
+    make(tma::kVxVyCentre, s->field[0], 2, 1, kTX, kTY);
+    make(tma::kVzCentre, s->field[2], 1, 1, kTX, kTY);
     cudaCheck(deviceMalloc(&s->maps, table.size() * sizeof(CUtensorMap)), "allocate tensor maps");
     cudaCheck(cudaMemcpyAsync(s->maps, table.data(), table.size() * sizeof(CUtensorMap), cudaMemcpyHostToDevice, s->stream),
               "upload tensor maps");

@@ -19,20 +19,25 @@ constexpr int kStages = 3;
 
 constexpr long long kWaitCycles = 4000000000LL;   // default wait limit, ~2 s at 1.9 GHz
 
-// Tensor-map table (one CUtensorMap per array and box shape), kept in global memory.
+// Tensor-map table, kept in global memory.  The twelve volumes of a session are equally spaced in
+// one allocation, so a four-dimensional map {x, y, z, volume} brings the tiles of several
+// fields (and, with a box two planes deep, of two planes) in one copy: 7 and 6 copies per stage
+// instead of 13 and 15, which the one issuing thread has to get out between two planes.
 enum MapIndex : int {
-    kCenter0 = 0,        // 0..8: field k, 32 x TY box; 9 = 1/rho, 10 = lambda, 11 = mu
-    kSxxX = 12,          // sigma_xx, (32+8) x TY (x halo)
-    kSxzX = 13,          // sigma_xz, (32+8) x TY
-    kSxyXY = 14,         // sigma_xy, (32+8) x (TY+8)
-    kSyyY = 15,          // sigma_yy, 32 x (TY+8)
-    kSyzY = 16,          // sigma_yz, 32 x (TY+8)
-    kVxXY = 17,          // vx, vy, vz: (32+8) x (TY+8)
-    kVyXY = 18,
-    kVzXY = 19,
-    kRhoT = 20,          // 1/rho, 36 x (TY+1)
-    kMuT = 21,           // mu, 36 x (TY+1)
-    kMapCount = 22
+    kSxxSxz = 0,         // sigma_xx and sigma_xz, (32+8) x TY (x halo)
+    kSxy = 1,            // sigma_xy, (32+8) x (TY+8)
+    kSyySyz = 2,         // sigma_yy and sigma_yz, 32 x (TY+8)
+    kRhoTwo = 3,         // 1/rho, 36 x (TY+1) x 2 planes
+    kVelocity = 4,       // vx, vy, vz, 32 x TY
+    kSyzSxzCentre = 5,   // sigma_yz and sigma_xz, 32 x TY
+    kSzzCentre = 6,      // sigma_zz, 32 x TY
+    kVelocityHalo = 7,   // vx, vy, vz, (32+8) x (TY+8)
+    kMuTwo = 8,          // mu, 36 x (TY+1) x 2 planes
+    kLambda = 9,         // lambda, 32 x TY
+    kStress = 10,        // the six stresses, 32 x TY
+    kVxVyCentre = 11,    // vx and vy, 32 x TY
+    kVzCentre = 12,      // vz, 32 x TY
+    kMapCount = 13
 };
 
 __device__ __forceinline__ uint32_t smemAddress(const void* p) {
@@ -82,11 +87,11 @@ __device__ __forceinline__ void fenceProxyAsync() {
     asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
 }
 
-// One 3-D tile copy global -> shared, completing on `bar`.
-__device__ __forceinline__ void load3d(void* dst, const CUtensorMap* map, int x, int y, int z, uint64_t* bar) {
+// One tile copy global -> shared from {x, y, z, first volume of the map}, completing on `bar`.
+__device__ __forceinline__ void load4d(void* dst, const CUtensorMap* map, int x, int y, int z, uint64_t* bar) {
     asm volatile(
-        "cp.async.bulk.tensor.3d.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3, %4}], [%5];"
-        ::"r"(smemAddress(dst)), "l"(reinterpret_cast<uint64_t>(map)), "r"(x), "r"(y), "r"(z), "r"(smemAddress(bar))
+        "cp.async.bulk.tensor.4d.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3, %4, %5}], [%6];"
+        ::"r"(smemAddress(dst)), "l"(reinterpret_cast<uint64_t>(map)), "r"(x), "r"(y), "r"(z), "r"(0), "r"(smemAddress(bar))
         : "memory");
 }
 
