@@ -221,16 +221,18 @@ struct seis3d_session {
     int device = 0;
     cudaStream_t stream = nullptr;
     int64_t pitch = 0, plane = 0;
-    float* pool = nullptr;          // 12 padded volumes: 9 fields, 3 materials
+    float* pool = nullptr;          // kLead elements, then 12 padded volumes: 9 fields, 3 materials
     std::size_t poolBytes = 0;
     float* field[9]{};
     float* invRho = nullptr;
     float* lambda = nullptr;
     float* mu = nullptr;
+    float* psiPool[3]{};            // kLead elements, then the CPML memories
     float* psi[3]{};                // CPML memories (FP32, or BF16 elements in SEIS3D_STORAGE_BF16_CPML)
     std::size_t psiCount[3]{};
     int storage = SEIS3D_STORAGE_FP32;
-    std::size_t psiBytes(int a) const { return psiCount[a] * (storage == SEIS3D_STORAGE_BF16_CPML ? 2 : 4); }
+    std::size_t memoryBytes() const { return storage == SEIS3D_STORAGE_BF16_CPML ? 2 : 4; }
+    std::size_t psiBytes(int a) const { return psiCount[a] * memoryBytes(); }
     float* coef[3]{};
     unsigned* status = nullptr;     // [0] non-finite flag, [1] staging stall
     unsigned* viewStats = nullptr;  // colour statistics of the view extraction (5 words)
@@ -321,7 +323,7 @@ void releaseSession(seis3d_session* s) noexcept {
     if (s->stream) cudaStreamSynchronize(s->stream);
     s->dropGraph();
     cudaFree(s->pool);
-    for (int a = 0; a < 3; ++a) { cudaFree(s->psi[a]); cudaFree(s->coef[a]); }
+    for (int a = 0; a < 3; ++a) { cudaFree(s->psiPool[a]); cudaFree(s->coef[a]); }
     cudaFree(s->status);
     cudaFree(s->viewStats);
     cudaFree(s->clock);
@@ -797,13 +799,13 @@ int seis3d_initialize(seis3d_session** out, const seis3d_context* context, const
             s->pitch = opt.compact_rows ? c.gx3D : roundUp(c.gx3D, 32);
             s->plane = s->pitch * c.gy3D;
             const std::size_t volume = std::size_t(s->plane) * c.gz3D;
-            s->poolBytes = volume * 12 * sizeof(float);
+            s->poolBytes = (kLead + volume * 12) * sizeof(float);
             cudaCheck(deviceMalloc(&s->pool, s->poolBytes), "allocate fields");
             cudaCheck(cudaMemsetAsync(s->pool, 0, s->poolBytes, s->stream), "clear fields");
-            for (int k = 0; k < 9; ++k) s->field[k] = s->pool + k * volume;
-            s->invRho = s->pool + 9 * volume;
-            s->lambda = s->pool + 10 * volume;
-            s->mu = s->pool + 11 * volume;
+            for (int k = 0; k < 9; ++k) s->field[k] = s->pool + kLead + k * volume;
+            s->invRho = s->pool + kLead + 9 * volume;
+            s->lambda = s->pool + kLead + 10 * volume;
+            s->mu = s->pool + kLead + 11 * volume;
             s->allocated = s->poolBytes;
             if (!c.reflecting3D) {
                 const int thick[3] = {2 * c.pml3D, 2 * c.pml3D, (c.freeSurface3D ? 1 : 2) * c.pml3D};
@@ -811,7 +813,10 @@ int seis3d_initialize(seis3d_session** out, const seis3d_context* context, const
                 s->psiCount[1] = std::size_t(6) * c.gz3D * thick[1] * s->pitch;
                 s->psiCount[2] = std::size_t(6) * thick[2] * c.gy3D * s->pitch;
                 for (int a = 0; a < 3; ++a) {
-                    cudaCheck(deviceMalloc(&s->psi[a], s->psiBytes(a)), "allocate CPML memories");
+                    // The x slab's rows are not x-pitched: its memories start at the allocation.
+                    const std::size_t lead = a == 0 ? 0 : kLead * s->memoryBytes();
+                    cudaCheck(deviceMalloc(&s->psiPool[a], lead + s->psiBytes(a)), "allocate CPML memories");
+                    s->psi[a] = s->psiPool[a] + lead / sizeof(float);
                     cudaCheck(cudaMemsetAsync(s->psi[a], 0, s->psiBytes(a), s->stream), "clear CPML");
                     s->allocated += s->psiBytes(a);
                     const auto k = coefficients(c, a);
@@ -856,7 +861,7 @@ int seis3d_reset(seis3d_session* s, const seis3d_context* c) {
         requireSession(s);
         requireSameGrid(s, c);
         const std::size_t volume = std::size_t(s->plane) * s->ctx.gz3D;
-        cudaCheck(cudaMemsetAsync(s->pool, 0, volume * 9 * sizeof(float), s->stream), "reset wavefield");
+        cudaCheck(cudaMemsetAsync(s->field[0], 0, volume * 9 * sizeof(float), s->stream), "reset wavefield");
         for (int a = 0; a < 3; ++a)
             if (s->psi[a]) cudaCheck(cudaMemsetAsync(s->psi[a], 0, s->psiBytes(a), s->stream), "reset CPML");
         cudaCheck(cudaMemsetAsync(s->status, 0, 4 * sizeof(unsigned), s->stream), "reset diagnostics");
