@@ -458,7 +458,7 @@ void configureKernels() {
 }
 
 // The pass kernels of a session's storage mode.
-using PassKernel = void (*)(Geometry, Fields, SourceParams, int);
+using PassKernel = void (*)(Geometry, Fields, SourceParams, StepParams);
 PassKernel velocityKernel(const seis3d_session* s) {
     return s->storage == SEIS3D_STORAGE_BF16_CPML ? velocityPassBf16Cpml : velocityPass;
 }
@@ -498,13 +498,24 @@ Shape passShape(const seis3d_session* s) {
     return sh;
 }
 
-// True when the passes write the free-surface images themselves: the first z chunk of each
-// pass writes those of its columns before its z rings read them, which needs chunks of at
-// least 4 planes (a shorter first chunk leaves ghost planes to the next chunk's rings).
-bool foldedImages(const Shape& sh) { return sh.zChunk >= kRadius; }
+// One pass; with `overlap` its set-up runs while the previous kernel of the stream, which has to
+// be a pass, drains (programmatic dependent launch).
+void launchPass(PassKernel kernel, const Shape& sh, std::size_t smem, cudaStream_t stream, bool overlap, const Geometry& G,
+                const Fields& F, const SourceParams& S, const StepParams& Q, const char* what) {
+    cudaLaunchAttribute attr{};
+    attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr.val.programmaticStreamSerializationAllowed = 1;
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = sh.grid;
+    cfg.blockDim = sh.block;
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = stream;
+    cfg.attrs = &attr;
+    cfg.numAttrs = overlap ? 1 : 0;
+    cudaCheck(cudaLaunchKernelEx(&cfg, kernel, G, F, S, Q), what);
+}
 
-// Slip-wall images of the velocities or the stresses, and with `surface` the free-surface
-// images (in a step only when the passes do not write them, foldedImages).
+// Slip-wall images of the velocities or the stresses, and with `surface` the free-surface images.
 void launchImages(seis3d_session* s, bool velocities, cudaStream_t stream = nullptr, bool surface = true) {
     const Geometry G = s->geometry();
     const Fields F = s->fields();
@@ -527,47 +538,62 @@ void launchImages(seis3d_session* s, bool velocities, cudaStream_t stream = null
     }
 }
 
-// One leapfrog step in the reference order (cuda/Cuda_Seis3D.cu:602-624), reading the
-// step index from the device clock; `leadingImages` re-applies the start-of-step slip-wall
-// stress images (idempotent after a previous step, needed after a reset or a field upload).
-// The free-surface stress images are written at the start of every velocity pass, where the
+// One leapfrog step in the reference order (cuda/Cuda_Seis3D.cu:602-624): the device clock's step
+// plus `slot`.  The velocity pass writes the free-surface stress images at its start, where the
 // reference's step starts with stressGhostKernel3D; its step also ends with them (:621), which
 // closingImages does once per API call (between the steps of a call nothing reads them).
+//
+// With `tail` (and always with the learned boundary, whose corrections come after the passes) a
+// tail kernel records the receivers and advances the clock after every step; else the stress
+// pass records them and the caller advances the clock past its steps (advance).  The tail
+// measured 2.5-3 us a step; a batch keeps it, where other shots' passes run beside it.
 // Optional events bracket the passes for seis3d_profile_steps.
 struct PassEvents { cudaEvent_t start, afterVelocity, afterImages, afterStress, end; };
 
 void enqueueBoundaryCorrection(seis3d_session* s, cudaStream_t stream);   // seis3d_boundary.inc
 
-void enqueueStep(seis3d_session* s, const SourceParams& S, bool leadingImages, const PassEvents* ev = nullptr,
+bool needsTail(const seis3d_session* s) { return s->net != nullptr; }
+
+void enqueueStep(seis3d_session* s, const SourceParams& S, int slot, bool tail, const PassEvents* ev = nullptr,
                  cudaStream_t stream = nullptr) {
     const Geometry G = s->geometry();
     const Fields F = s->fields();
     const Shape sh = passShape(s);
     if (!stream) stream = s->stream;
-    const bool folded = foldedImages(sh);
-    if (leadingImages) launchImages(s, false, stream);
+    float* gather = s->gatherActive ? s->gather : nullptr;
+    const StepParams Q{sh.zChunk, tail ? 0 : slot, s->recv, s->recvCount, tail ? nullptr : gather};
     if (ev) cudaEventRecord(ev->start, stream);
-    velocityKernel(s)<<<sh.grid, sh.block, kVelocitySmem, stream>>>(G, F, S, sh.zChunk);
-    launchCheck("velocity pass");
+    launchPass(velocityKernel(s), sh, kVelocitySmem, stream, !ev && !tail && slot > 0, G, F, S, Q, "velocity pass");
     ++s->launches;
     if (ev) cudaEventRecord(ev->afterVelocity, stream);
-    launchImages(s, true, stream, !folded);
+    launchImages(s, true, stream, false);
     if (ev) cudaEventRecord(ev->afterImages, stream);
-    stressKernel(s)<<<sh.grid, sh.block, kStressSmem, stream>>>(G, F, S, sh.zChunk);
-    launchCheck("stress pass");
+    launchPass(stressKernel(s), sh, kStressSmem, stream, !ev, G, F, S, Q, "stress pass");
     ++s->launches;
     if (ev) cudaEventRecord(ev->afterStress, stream);
-    launchImages(s, false, stream, !folded || s->net != nullptr);
+    launchImages(s, false, stream, s->net != nullptr);
     if (s->net) {
         // Learned thin boundary: corrections of the boundary columns after the full step (on
         // the imaged state), then the stress images again for the corrected cells.
         enqueueBoundaryCorrection(s, stream);
         launchImages(s, false, stream);
     }
-    stepTail<<<1, 256, 0, stream>>>(G, F, s->recv, s->recvCount, s->gatherActive ? s->gather : nullptr);
-    launchCheck("step tail");
-    ++s->launches;
+    if (tail) {
+        stepTail<<<1, 256, 0, stream>>>(G, F, s->recv, s->recvCount, gather);
+        launchCheck("step tail");
+        ++s->launches;
+    }
     if (ev) cudaEventRecord(ev->end, stream);
+}
+
+// `steps` steps from the clock's and the clock past them.
+void enqueueSteps(seis3d_session* s, const SourceParams& S, int steps) {
+    const bool tail = needsTail(s);
+    for (int k = 0; k < steps; ++k) enqueueStep(s, S, k, tail);
+    if (tail || steps == 0) return;
+    advanceClock<<<1, 1, 0, s->stream>>>(s->clock, steps, s->gatherActive ? 1 : 0);
+    launchCheck("advance clock");
+    ++s->launches;
 }
 
 // The free-surface stress images after the last step of an API call, so that the state
@@ -602,9 +628,9 @@ void tuneZChunk(seis3d_session* s) {
             s->zChunk = z;
             const Shape sh = passShape(s);
             auto pair = [&] {
-                velocityKernel(s)<<<sh.grid, sh.block, kVelocitySmem, s->stream>>>(G, F, S, sh.zChunk);
-                stressKernel(s)<<<sh.grid, sh.block, kStressSmem, s->stream>>>(G, F, S, sh.zChunk);
-                launchCheck("z chunk tuning");
+                const StepParams Q{sh.zChunk, 0, nullptr, 0, nullptr};
+                launchPass(velocityKernel(s), sh, kVelocitySmem, s->stream, false, G, F, S, Q, "z chunk tuning");
+                launchPass(stressKernel(s), sh, kStressSmem, s->stream, true, G, F, S, Q, "z chunk tuning");
                 s->launches += 2;
             };
             pair();
@@ -909,7 +935,8 @@ int seis3d_run_step(seis3d_session* s, const seis3d_context* c, const seis3d_sou
         requireSameGrid(s, c);
         adoptScalars(s, c);
         syncClock(s, step);
-        enqueueStep(s, sourceParams(s->ctx, *src), true);
+        launchImages(s, false);
+        enqueueSteps(s, sourceParams(s->ctx, *src), 1);
         closingImages(s);
         s->hostClock = step + 1;
     });
@@ -928,7 +955,7 @@ static void ensureGraph(seis3d_session* s, const seis3d_source& src, const Sourc
     const uint64_t before = s->launches;
     cudaCheck(cudaStreamBeginCapture(s->stream, cudaStreamCaptureModeThreadLocal), "begin capture");
     try {
-        for (int k = 0; k < kGraphBatch; ++k) enqueueStep(s, S, false);
+        enqueueSteps(s, S, kGraphBatch);
     } catch (...) {
         cudaStreamEndCapture(s->stream, &g);
         if (g) cudaGraphDestroy(g);
@@ -968,7 +995,7 @@ int seis3d_run_steps(seis3d_session* s, const seis3d_context* c, const seis3d_so
                 s->launches += s->graphNodes;
             }
         }
-        for (; done < count; ++done) enqueueStep(s, S, false);
+        enqueueSteps(s, S, count - done);
         closingImages(s);
         s->hostClock = first + uint64_t(count);
     });
@@ -1315,7 +1342,7 @@ int seis3d_profile_steps(seis3d_session* s, const seis3d_context* c, const seis3
         for (auto& e : ev)
             for (cudaEvent_t* p : {&e.start, &e.afterVelocity, &e.afterImages, &e.afterStress, &e.end})
                 cudaCheck(cudaEventCreate(p), "create event");
-        for (int k = 0; k < count; ++k) enqueueStep(s, S, false, &ev[std::size_t(k)]);
+        for (int k = 0; k < count; ++k) enqueueStep(s, S, 0, true, &ev[std::size_t(k)]);
         closingImages(s);
         s->hostClock = first + uint64_t(count);
         cudaCheck(cudaStreamSynchronize(s->stream), "profile steps");

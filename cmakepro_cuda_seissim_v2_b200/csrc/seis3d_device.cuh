@@ -63,9 +63,18 @@ struct SourceParams {
     float direction[3];
 };
 
+// One step of a pass as its launch gives it.
+struct StepParams {
+    int zChunk;            // planes per CTA
+    int slot;              // steps since the clock's: the step executed is clock->step + slot
+    const int4* receivers; // grid coordinates; sampled by the stress pass when `gather` is set
+    int receiverCount;
+    float* gather;         // [sample][receiver][3], or null
+};
+
 // Device clock and gather state shared by the kernels of one session.
 struct Clock {
-    unsigned long long step;   // time index of the step being executed
+    unsigned long long step;   // time index of the first step of the running batch
     int sample;                // samples recorded so far in the active gather
     int stride;                // gather stride (0 = no active gather)
     int target;                // samples to record

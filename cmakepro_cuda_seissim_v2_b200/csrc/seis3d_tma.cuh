@@ -81,6 +81,15 @@ __device__ __forceinline__ bool waitStage(uint64_t* bar, uint32_t parity, long l
     return true;
 }
 
+// Programmatic dependent launch: the next kernel of the stream may become resident as soon as
+// every CTA has called launchDependents, and waits in waitForPrevious until this one has
+// completed and its writes are visible.  Both are no-ops in an ordinary launch.  A CTA calls
+// the first after its last plane: with the call at its start, the next pass's CTAs sat waiting
+// in the slots beside it, and the 40x32x36 step took 33.9 us instead of 28.6 (30.8 without
+// programmatic launch).
+__device__ __forceinline__ void launchDependents() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+__device__ __forceinline__ void waitForPrevious() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+
 // Order this thread's earlier generic-proxy shared-memory accesses before its later
 // async-proxy (TMA) accesses.
 __device__ __forceinline__ void fenceProxyAsync() {
