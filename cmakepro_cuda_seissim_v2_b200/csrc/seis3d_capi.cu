@@ -498,44 +498,57 @@ Shape passShape(const seis3d_session* s) {
     return sh;
 }
 
-// One pass; with `overlap` its set-up runs while the previous kernel of the stream, which has to
-// be a pass, drains (programmatic dependent launch).
+// A launch; with `overlap` its set-up runs while the previous kernel of the stream drains
+// (programmatic dependent launch), which is for kernels that call tma::waitForPrevious.
+struct Overlapped {
+    cudaLaunchAttribute attr{};
+    cudaLaunchConfig_t cfg{};
+    Overlapped(dim3 grid, dim3 block, std::size_t smem, cudaStream_t stream, bool overlap) {
+        attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+        attr.val.programmaticStreamSerializationAllowed = 1;
+        cfg.gridDim = grid;
+        cfg.blockDim = block;
+        cfg.dynamicSmemBytes = smem;
+        cfg.stream = stream;
+        cfg.attrs = &attr;
+        cfg.numAttrs = overlap ? 1 : 0;
+    }
+    Overlapped(const Overlapped&) = delete;
+    Overlapped& operator=(const Overlapped&) = delete;
+};
+
 void launchPass(PassKernel kernel, const Shape& sh, std::size_t smem, cudaStream_t stream, bool overlap, const Geometry& G,
                 const Fields& F, const SourceParams& S, const StepParams& Q, const char* what) {
-    cudaLaunchAttribute attr{};
-    attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    attr.val.programmaticStreamSerializationAllowed = 1;
-    cudaLaunchConfig_t cfg{};
-    cfg.gridDim = sh.grid;
-    cfg.blockDim = sh.block;
-    cfg.dynamicSmemBytes = smem;
-    cfg.stream = stream;
-    cfg.attrs = &attr;
-    cfg.numAttrs = overlap ? 1 : 0;
-    cudaCheck(cudaLaunchKernelEx(&cfg, kernel, G, F, S, Q), what);
+    const Overlapped launch(sh.grid, sh.block, smem, stream, overlap);
+    cudaCheck(cudaLaunchKernelEx(&launch.cfg, kernel, G, F, S, Q), what);
 }
 
-// Slip-wall images of the velocities or the stresses, and with `surface` the free-surface images.
-void launchImages(seis3d_session* s, bool velocities, cudaStream_t stream = nullptr, bool surface = true) {
-    const Geometry G = s->geometry();
-    const Fields F = s->fields();
+// Images of the velocities or the stresses at the free surface (in a step the passes write those
+// they read themselves).
+void launchSurfaceImages(seis3d_session* s, bool velocities, cudaStream_t stream) {
+    if (!s->ctx.freeSurface3D) return;
+    const dim3 b(32, 8), g((s->ctx.gx3D - 8 + 31) / 32, (s->ctx.gy3D - 8 + 7) / 8);
+    if (velocities) velocityImages<<<g, b, 0, stream>>>(s->geometry(), s->fields());
+    else stressImages<<<g, b, 0, stream>>>(s->geometry(), s->fields());
+    launchCheck("free-surface images");
+    ++s->launches;
+}
+
+// Images of the velocities or the stresses of the slip walls; `overlap` as in launchPass.
+void launchWallImages(seis3d_session* s, bool velocities, cudaStream_t stream, bool overlap) {
+    if (!s->ctx.reflecting3D) return;
+    const int gx = s->ctx.gx3D, gy = s->ctx.gy3D, gz = s->ctx.gz3D, shell = 2 * kRadius + 1;
+    const int cells = shell * (gx * gy + gx * (gz - shell) + (gy - shell) * (gz - shell));
+    const Overlapped launch(dim3((cells + 255) / 256), dim3(256), 0, stream, overlap);
+    cudaCheck(cudaLaunchKernelEx(&launch.cfg, velocities ? wallImages<true> : wallImages<false>, s->geometry(), s->fields()),
+              "wall images");
+    ++s->launches;
+}
+
+void launchImages(seis3d_session* s, bool velocities, cudaStream_t stream = nullptr) {
     if (!stream) stream = s->stream;
-    if (s->ctx.freeSurface3D && surface) {
-        const dim3 b(32, 8), g((s->ctx.gx3D - 8 + 31) / 32, (s->ctx.gy3D - 8 + 7) / 8);
-        if (velocities) velocityImages<<<g, b, 0, stream>>>(G, F);
-        else stressImages<<<g, b, 0, stream>>>(G, F);
-        launchCheck("free-surface images");
-        ++s->launches;
-    }
-    if (s->ctx.reflecting3D) {
-        const int len[3] = {s->ctx.gx3D, s->ctx.gy3D, s->ctx.gz3D};
-        for (int axis = 0; axis < 3; ++axis) {
-            const dim3 b(16, 16), g((len[(axis + 1) % 3] + 15) / 16, (len[(axis + 2) % 3] + 15) / 16);
-            reflectingImages<<<g, b, 0, stream>>>(G, F, axis, velocities ? 1 : 0);
-            launchCheck("reflecting images");
-            ++s->launches;
-        }
-    }
+    launchSurfaceImages(s, velocities, stream);
+    launchWallImages(s, velocities, stream, false);
 }
 
 // One leapfrog step in the reference order (cuda/Cuda_Seis3D.cu:602-624): the device clock's step
@@ -566,13 +579,14 @@ void enqueueStep(seis3d_session* s, const SourceParams& S, int slot, bool tail, 
     launchPass(velocityKernel(s), sh, kVelocitySmem, stream, !ev && !tail && slot > 0, G, F, S, Q, "velocity pass");
     ++s->launches;
     if (ev) cudaEventRecord(ev->afterVelocity, stream);
-    launchImages(s, true, stream, false);
+    launchWallImages(s, true, stream, !ev);
     if (ev) cudaEventRecord(ev->afterImages, stream);
     launchPass(stressKernel(s), sh, kStressSmem, stream, !ev, G, F, S, Q, "stress pass");
     ++s->launches;
     if (ev) cudaEventRecord(ev->afterStress, stream);
-    launchImages(s, false, stream, s->net != nullptr);
+    launchWallImages(s, false, stream, !ev);
     if (s->net) {
+        launchSurfaceImages(s, false, stream);
         // Learned thin boundary: corrections of the boundary columns after the full step (on
         // the imaged state), then the stress images again for the corrected cells.
         enqueueBoundaryCorrection(s, stream);
