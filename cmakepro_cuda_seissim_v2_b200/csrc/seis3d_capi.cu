@@ -469,28 +469,42 @@ PassKernel stressKernel(const seis3d_session* s) {
 // Launch shapes of the two passes.
 struct Shape { dim3 grid, block; int zChunk; };
 
-Shape passShape(const seis3d_session* s) {
+// Time of a pass over `planes` planes cut into chunks of c, in units of one plane of one CTA when
+// the device is full: what CTAs of `tiles` tiles cost on `slots` resident places.
+//   * Up to one CTA per SM (half the places) a CTA has its SM to itself: 0.7 of the full time per
+//     plane, and 2 planes' worth of start (rings, first stages, launch).  With the second CTA of
+//     an SM the time per plane grows to the full one.
+//   * Beyond one round of places the work is shared evenly and a CTA's start is mostly hidden
+//     behind its neighbour (0.8 planes), but the last CTAs to finish leave the device part empty
+//     for `tail` of a CTA's time: nine tenths when nothing runs beside the pass, nothing in a
+//     batch, where other shots fill it (three windows of 161x120x171 to 205x97x160: 649 us a
+//     step with 20-plane chunks, 681 with 8).
+// Fitted to the step times of 16 grids from 40x32x36 to 300x300x400 with chunks of 2 to 24
+// planes; the chunk it picks is within 1.7 % of the best one on average (5.6 % at most).  The
+// former rule (18 to 32 planes, whole rounds of places) left small grids to a few SMs:
+// 40x32x36 85.7 us a step against 24.1, 97x61x83 between walls 68.1 against 25.7, 161x120x171
+// with 20-cell CPML 260.8 against 229.2, 300x300x400 1334 against 1277.
+double passTime(int tiles, int planes, int c, double slots, double tail) {
+    const double rounds = tiles * double((planes + c - 1) / c) / slots;
+    if (rounds <= 0.5) return 0.7 * (c + 2);
+    if (rounds <= 1.0) return (0.7 + 0.3 * (2 * rounds - 1)) * (c + 2);
+    return (c + 0.8) * (rounds + tail * std::min(1.0, rounds - 1)) + 1.2;
+}
+
+// `concurrent` sessions of a batch step together, each with its share of the places.
+Shape passShape(const seis3d_session* s, int concurrent = 1) {
     const int nxA = s->ctx.gx3D - 8, nyA = s->ctx.gy3D - 8, nzA = s->ctx.gz3D - 8;
     const int tilesX = (nxA + kTX - 1) / kTX, tilesY = (nyA + kTY - 1) / kTY;
-    const int tiles = tilesX * tilesY;
-    int chunks = 1;
-    if (s->zChunk > 0) {
-        chunks = (nzA + s->zChunk - 1) / s->zChunk;
-    } else {
-        // Chunks of 18-32 planes (measured best on B200: many CTAs per SM over the run
-        // keep the HBM streams spread), picking the split that fills whole waves of the
-        // resident CTA slots best, with each chunk's 7-plane ring warm-up as overhead.
-        const double slots = double(std::max(1, s->residentCtas));
-        double best = -1.0;
-        const int lo = std::max(1, nzA / 32), hi = std::max(lo, nzA / 18);
-        for (int n = lo; n <= hi; ++n) {
-            const double waves = tiles * double(n) / slots;
-            const double fill = waves / std::ceil(waves);
-            const double chunk = std::ceil(double(nzA) / n);
-            const double score = fill * chunk / (chunk + 7.0);
-            if (score > best + 1e-9) { best = score; chunks = n; }
+    int chunk = s->zChunk;
+    if (chunk <= 0) {
+        const double slots = double(std::max(1, s->residentCtas)) / concurrent;
+        double best = std::numeric_limits<double>::max();
+        for (int c = 2; c <= 24; ++c) {
+            const double t = passTime(tilesX * tilesY, nzA, c, slots, concurrent > 1 ? 0.0 : 0.9);
+            if (t < best - 1e-9) { best = t; chunk = c; }
         }
     }
+    const int chunks = (nzA + chunk - 1) / chunk;
     Shape sh;
     sh.zChunk = (nzA + chunks - 1) / chunks;
     sh.block = dim3(kTX, kWarps);
@@ -568,10 +582,10 @@ void enqueueBoundaryCorrection(seis3d_session* s, cudaStream_t stream);   // sei
 bool needsTail(const seis3d_session* s) { return s->net != nullptr; }
 
 void enqueueStep(seis3d_session* s, const SourceParams& S, int slot, bool tail, const PassEvents* ev = nullptr,
-                 cudaStream_t stream = nullptr) {
+                 cudaStream_t stream = nullptr, int concurrent = 1) {
     const Geometry G = s->geometry();
     const Fields F = s->fields();
-    const Shape sh = passShape(s);
+    const Shape sh = passShape(s, concurrent);
     if (!stream) stream = s->stream;
     float* gather = s->gatherActive ? s->gather : nullptr;
     const StepParams Q{sh.zChunk, tail ? 0 : slot, s->recv, s->recvCount, tail ? nullptr : gather};
