@@ -727,6 +727,25 @@ void buildTensorMaps(seis3d_session* s) {
     cudaCheck(cudaStreamSynchronize(s->stream), "upload tensor maps");
 }
 
+// The extraction kernel of a wave and a material component.  Components 5-7 ask for a material
+// as the wave (sampleScalar3D takes one range of components).
+using ViewKernel = void (*)(ViewArgs, unsigned);
+template <int kWave> ViewKernel viewKernelOf(int material) {
+    return material == 5 ? extractViews<kWave, 5> : material == 6 ? extractViews<kWave, 6> : extractViews<kWave, 7>;
+}
+ViewKernel viewKernel(int wave, int material) {
+    switch (wave) {
+        case 0: return viewKernelOf<0>(material);
+        case 1: return viewKernelOf<1>(material);
+        case 2: return viewKernelOf<2>(material);
+        case 3: return viewKernelOf<3>(material);
+        case 4: return viewKernelOf<4>(material);
+        case 5: return viewKernelOf<5>(material);
+        case 6: return viewKernelOf<6>(material);
+        default: return viewKernelOf<7>(material);
+    }
+}
+
 }  // namespace
 
 // --------------------------------------------------------------------------------------
@@ -1445,7 +1464,9 @@ int seis3d_extract_views(seis3d_session* s, const seis3d_context* c, float* outp
         a.stats = s->viewStats;
         a.nonFinite = s->status;
         if (count > 0) {
-            extractViews<<<unsigned((count + 255) / 256), 256, 0, s->stream>>>(a, count);
+            // Blocks for eight to run on every SM; each strides over its share of the samples.
+            const uint64_t blocks = std::min<uint64_t>((count + kViewThreads - 1) / kViewThreads, uint64_t(s->smCount) * 8);
+            viewKernel(component, material_component)<<<unsigned(blocks), kViewThreads, 0, s->stream>>>(a, unsigned(count));
             launchCheck("extract views");
             ++s->launches;
         }
