@@ -228,18 +228,32 @@ struct seis2d_session {
 
 namespace {
 
-dim3 stressGrid(const Grid2D& g) { return dim3((g.NX + kBX - 1) / kBX, (g.NZ + kBY - 1) / kBY + 1); }
-dim3 velocityGrid(const Grid2D& g) { return dim3((g.NX + kBX - 1) / kBX, (g.NZ + kBY - 1) / kBY); }
-const dim3 kBlock(kBX, kBY);
+// One strip per block, and for the stresses a row of blocks that samples the receivers.
+dim3 stressGrid(const Grid2D& g, int scheme, int rows) { return dim3(stripsAcross(g), stressStrips(g, scheme, rows) + 1); }
+dim3 velocityGrid(const Grid2D& g, int rows) { return dim3(stripsAcross(g), velocityStrips(g, rows)); }
 constexpr int kSourceThreads = 256;
 constexpr int kGraphBatch = 64;
 static_assert(kSourceThreads >= SEIS2D_MAX_ACTIVE_SOURCES, "one thread per active source");
 
-template <int S> void launchStress(seis2d_session* s, int slot) {
-    stressStep<S><<<stressGrid(s->g), kBlock, 0, s->stream>>>(s->g, s->f, s->ctl, slot);
+// A step kernel; with `overlap` it is launched while the previous kernel of the stream drains
+// (programmatic dependent launch; both step kernels wait for that one before they read).
+template <class K> void launchStep(K kernel, dim3 grid, seis2d_session* s, int slot, bool overlap) {
+    cudaLaunchAttribute attr{};
+    attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr.val.programmaticStreamSerializationAllowed = 1;
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = grid;
+    cfg.blockDim = dim3(kThreads);
+    cfg.stream = s->stream;
+    cfg.attrs = &attr;
+    cfg.numAttrs = overlap ? 1 : 0;
+    cudaCheck(cudaLaunchKernelEx(&cfg, kernel, s->g, s->f, static_cast<const Control2D*>(s->ctl), slot), "step kernel launch");
 }
-template <int S> void launchVelocity(seis2d_session* s, int slot) {
-    velocityStep<S><<<velocityGrid(s->g), kBlock, 0, s->stream>>>(s->g, s->f, s->ctl, slot);
+template <int S, int R> void launchStress(seis2d_session* s, int slot, bool overlap) {
+    launchStep(stressStep<S, R>, stressGrid(s->g, S, R), s, slot, overlap);
+}
+template <int S, int R> void launchVelocity(seis2d_session* s, int slot, bool overlap) {
+    launchStep(velocityStep<S, R>, velocityGrid(s->g, R), s, slot, overlap);
 }
 template <int S> void launchInject(seis2d_session* s) {
     injectSources<S><<<1, kSourceThreads, 0, s->stream>>>(s->g, s->f, s->ctl);
@@ -254,13 +268,23 @@ template <class F> void dispatch(int scheme, F&& fn) {
     else fn(std::integral_constant<int, kSplit>{});
 }
 
+// fn with the session's scheme and the rows of its strips as constants.
+template <class F> void dispatchStep(const seis2d_session* s, F&& fn) {
+    dispatch(s->scheme, [&](auto scheme) {
+        const int rows = stripRows(s->g.total);
+        if (rows == 1) fn(scheme, std::integral_constant<int, 1>{});
+        else if (rows == 2) fn(scheme, std::integral_constant<int, 2>{});
+        else fn(scheme, std::integral_constant<int, 3>{});
+    });
+}
+
 // Enqueues `batch` steps (graph slots 0..batch-1) and the batch end.
 void enqueueBatch(seis2d_session* s, int batch, bool multi) {
-    dispatch(s->scheme, [&](auto tag) {
-        constexpr int S = decltype(tag)::value;
+    dispatchStep(s, [&](auto tag, auto rows) {
+        constexpr int S = decltype(tag)::value, R = decltype(rows)::value;
         for (int slot = 0; slot < batch; ++slot) {
-            launchStress<S>(s, slot);
-            launchVelocity<S>(s, slot);
+            launchStress<S, R>(s, slot, slot > 0 && !multi);
+            launchVelocity<S, R>(s, slot, true);
             if (multi) launchInject<S>(s);
         }
         launchFinish<S>(s, batch - 1, batch);
@@ -270,23 +294,23 @@ void enqueueBatch(seis2d_session* s, int batch, bool multi) {
 }
 
 // Blocks of the persistent kernel that fit on the device at once (cooperative launch bound).
-template <int S> int residentBlocks() {
+template <int S, int R> int residentBlocks() {
     int device = 0, sms = 0, perSm = 0;
     cudaCheck(cudaGetDevice(&device), "device");
     cudaCheck(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device), "SM count");
-    cudaCheck(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&perSm, runSteps<S>, kThreads, 0), "occupancy");
+    cudaCheck(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&perSm, runSteps<S, R>, kThreads, 0), "occupancy");
     return perSm * sms;
 }
 
 // One cooperative launch of `count` steps (after configure()).
 void launchPersistent(seis2d_session* s, int count) {
-    const int tiles = ((s->g.NX + kBX - 1) / kBX) * ((s->g.NZ + kBY - 1) / kBY);
-    const int blocks = std::min(tiles, s->persistentBlocks);
+    const int strips = stripsAcross(s->g) * velocityStrips(s->g, stripRows(s->g.total));
+    const int blocks = std::min(strips, s->persistentBlocks);
     cudaCheck(cudaMemsetAsync(s->gridSync, 0, sizeof(GridSync), s->stream), "clear grid barrier");
-    dispatch(s->scheme, [&](auto tag) {
-        constexpr int S = decltype(tag)::value;
+    dispatchStep(s, [&](auto tag, auto rows) {
+        constexpr int S = decltype(tag)::value, R = decltype(rows)::value;
         void* args[] = {&s->g, &s->f, &s->ctl, &s->gridSync, &count, &s->barrier};
-        cudaCheck(cudaLaunchCooperativeKernel(reinterpret_cast<void*>(runSteps<S>), dim3(blocks), kBlock, args, 0,
+        cudaCheck(cudaLaunchCooperativeKernel(reinterpret_cast<void*>(runSteps<S, R>), dim3(blocks), dim3(kThreads), args, 0,
                                               s->stream),
                   "persistent launch");
     });
@@ -702,7 +726,10 @@ int seis2d_initialize(seis2d_session** session, const seis2d_context* context) {
             int cooperative = 0, device = 0;
             cudaCheck(cudaGetDevice(&device), "device");
             cudaCheck(cudaDeviceGetAttribute(&cooperative, cudaDevAttrCooperativeLaunch, device), "cooperative launch");
-            if (cooperative) dispatch(s->scheme, [&](auto tag) { s->persistentBlocks = residentBlocks<decltype(tag)::value>(); });
+            if (cooperative)
+                dispatchStep(s, [&](auto tag, auto rows) {
+                    s->persistentBlocks = residentBlocks<decltype(tag)::value, decltype(rows)::value>();
+                });
             s->sync();
             *session = s;
             const int status = seis2d_update_receivers(s, c.rcv_grid_idx.data, c.num_rcv);
@@ -992,15 +1019,15 @@ int seis2d_profile_steps(seis2d_session* session, int first_it, int count, const
         std::vector<cudaEvent_t> ev(std::size_t(count) * 3 + 1);
         for (auto& e : ev) cudaCheck(cudaEventCreate(&e), "event");
         try {
-            dispatch(s->scheme, [&](auto tag) {
-                constexpr int S = decltype(tag)::value;
+            dispatchStep(s, [&](auto tag, auto rows) {
+                constexpr int S = decltype(tag)::value, R = decltype(rows)::value;
                 for (int q = 0; q < count; ++q) {
                     // Each step is its own batch of one, so slot 0 and the batch end keep the
                     // field state of the reference after every step.
                     cudaEventRecord(ev[3 * q], s->stream);
-                    launchStress<S>(s, 0);
+                    launchStress<S, R>(s, 0, false);
                     cudaEventRecord(ev[3 * q + 1], s->stream);
-                    launchVelocity<S>(s, 0);
+                    launchVelocity<S, R>(s, 0, false);
                     cudaEventRecord(ev[3 * q + 2], s->stream);
                     launchFinish<S>(s, 0, 1);
                 }

@@ -31,13 +31,21 @@
 
 namespace seis2d {
 
-constexpr int kBX = 32;               // threads along x per block (one warp per row)
-constexpr int kBY = 16;               // rows per block
-constexpr int kThreads = kBX * kBY;   // one cell per thread
+// Programmatic dependent launch: a step kernel may become resident once every block of the one
+// before it has called launchDependents, and waits in waitForPrevious until that one has
+// completed.  Both are no-ops in an ordinary launch.
+__device__ __forceinline__ void launchDependents() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+__device__ __forceinline__ void waitForPrevious() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+
+constexpr int kThreads = 128;         // columns a block loads, one per thread
 constexpr int kHalo = 4;              // stencil radius (kStencilRadius, SolverNumerics.h:9)
-constexpr int kTW = kBX + 2 * kHalo;  // tile width
-constexpr int kTH = kBY + 2 * kHalo;  // tile height
-constexpr int kTile = kTW * kTH;
+constexpr int kCols = kThreads - 2 * kHalo;   // columns a block updates
+
+// Rows a thread updates, 1 to 3.  More rows mean fewer halo rows read per cell (R + 7 for R), fewer
+// rows more blocks and a shorter chain in each: us a step of 1 / 2 / 3 / 4 rows on 120x100 4.5 / 5.2
+// / 6.0 / 7.0, 250x300 7.2 / 7.0 / 7.4 / 8.9, 440x420 11.4 / 10.3 / 9.5 / 9.9, 1601x1203 88 /
+// 75 / 69 / 78 (split halves; the hybrid scheme has the same order).
+__host__ __device__ __forceinline__ int stripRows(int cells) { return cells <= 40000 ? 1 : cells <= 100000 ? 2 : 3; }
 
 // Scheme ids of the kernels (flag_type, with flag 3 and upFlag off run as flag 1;
 // Cuda_Check.cu:1038-1046).
@@ -81,70 +89,208 @@ struct Control2D {
     seis2d_source* sources;
 };
 
-// ---- shared-memory tiles ----------------------------------------------------------------
+// ---- strips ------------------------------------------------------------------------------
+//
+// A block updates R rows of kCols columns (stripRows).  A thread owns one column: it loads the rows its
+// z derivatives span straight into registers (R + 7 per array) and shares only its own rows
+// through shared memory for its neighbours' x derivatives; the first and last four threads only
+// share.  All loads (the cells' own values and materials too) are issued before the one
+// barrier, so a block waits for memory once.
 
-// Tile of a field around the block: rows i0-4 .. i0+kBY+3, columns j0-4 .. j0+kBX+3; cells
-// outside the grid read 0 (no computed cell uses them).
-struct TileRef {
-    float (*t)[kTW];
-    __device__ __forceinline__ float operator()(int di, int dj) const {
-        return t[threadIdx.y + kHalo + di][threadIdx.x + kHalo + dj];
+// One array of a strip as its thread holds it: rows first .. first + R + 6 of its column.
+template <int R> struct Column {
+    float v[R + 7];
+    __device__ __forceinline__ void load(const float* f, const Grid2D& g, int first, int j) {
+#pragma unroll
+        for (int k = 0; k < R + 7; ++k) {
+            const int i = first + k;
+            // L2-only loads: in a persistent run other blocks rewrite these fields between the
+            // grid barriers, so neither the read-only path nor L1 may hold an old copy.
+            v[k] = i < g.NZ ? __ldcg(f + i * g.NX + j) : 0.0f;
+        }
+    }
+    // The thread's own rows only, where they stand in a column that starts `before` rows earlier.
+    __device__ __forceinline__ void loadOwn(const float* f, const Grid2D& g, int row, int j, int before) {
+#pragma unroll
+        for (int r = 0; r < R; ++r) v[before + r] = row + r < g.NZ ? __ldcg(f + (row + r) * g.NX + j) : 0.0f;
     }
 };
 
-__device__ __forceinline__ void loadTiles(const Grid2D& g, int i0, int j0, float* dst, const float* const* src,
-                                          int count) {
-    const int tid = threadIdx.y * kBX + threadIdx.x;
-    for (int t = tid; t < kTile; t += kThreads) {
-        const int r = t / kTW, c = t - (t / kTW) * kTW;
-        const int i = i0 - kHalo + r, j = j0 - kHalo + c;
-        const bool in = i >= 0 && i < g.NZ && j >= 0 && j < g.NX;
-        const int k = i * g.NX + j;
-        // L2-only loads: in a persistent run other blocks rewrite these fields between the
-        // grid barriers, so neither the read-only path nor L1 may hold an old copy.
-        for (int a = 0; a < count; ++a) dst[a * kTile + t] = in ? __ldcg(src[a] + k) : 0.0f;
-    }
+using Shared = float[kThreads];   // one row of one array across the block
+
+// Weighted sum of four taps, in the reference's order.  The roundings that the compiler's
+// contraction gives the reference's expression are written out, here and in advance, so that
+// the results do not depend on how the surrounding code is arranged.
+__device__ __forceinline__ float weigh(const Grid2D& g, float t1, float t2, float t3, float t4) {
+    return __fmaf_rn(g.c4, t4, __fmaf_rn(g.c3, t3, __fmaf_rn(g.c1, t1, __fmul_rn(g.c2, t2))));
 }
 
-// Split-field first derivatives, written exactly as the reference kernels write them
-// (Cuda_Check.cu:236-254, 283-304, 434-486, 530-559): for each tap the two halves of the
-// upper sample, minus the two halves of the lower sample.
-struct Split {
-    TileRef a, b;
-    __device__ __forceinline__ float tap(int ui, int uj, int li, int lj) const {
-        return a(ui, uj) + b(ui, uj) - a(li, lj) - b(li, lj);
+struct Damp;
+// Damping of the thread's column and rows, loaded with everything else: between the rows' stores
+// each of these loads would wait for memory on its own.
+template <int R> struct Damping {
+    float x, xh, z[R], zh[R];
+    __device__ __forceinline__ void load(const Grid2D& g, const Fields2D& f, int row, int j) {
+        x = f.dx[j]; xh = f.dxh[j];
+#pragma unroll
+        for (int r = 0; r < R; ++r) {
+            const int i = min(row + r, g.NZ - 1);
+            z[r] = f.dz[i]; zh[r] = f.dzh[i];
+        }
     }
+    // Of own row r; `undamped` rows near a free surface have no damping along z.
+    __device__ __forceinline__ Damp at(int r, bool undamped) const;
 };
 
-// Forward x derivative (samples j+1..j+4 minus j..j-3).
-__device__ __forceinline__ float dxForward(const Grid2D& g, const Split& f) {
-    return g.c1 * f.tap(0, 1, 0, 0) + g.c2 * f.tap(0, 2, 0, -1) + g.c3 * f.tap(0, 3, 0, -2) + g.c4 * f.tap(0, 4, 0, -3);
+// One split half: (old (1/dt - d) + m D) / (1/dt + d).
+__device__ __forceinline__ float advance(const Grid2D& g, float old, float d, float m, float derivative) {
+    return __fmaf_rn(old, g.inv_dt - d, __fmul_rn(m, derivative)) / (g.inv_dt + d);
 }
-// Backward x derivative (samples j..j+3 minus j-1..j-4).
-__device__ __forceinline__ float dxBackward(const Grid2D& g, const Split& f) {
-    return g.c1 * f.tap(0, 0, 0, -1) + g.c2 * f.tap(0, 1, 0, -2) + g.c3 * f.tap(0, 2, 0, -3) + g.c4 * f.tap(0, 3, 0, -4);
+
+// Split-field first derivatives (Cuda_Check.cu:236-254, 283-304, 434-486, 530-559): each tap is the
+// two halves of the upper sample minus the two halves of the lower sample, in that order, so the
+// sum of the upper halves is formed once per sample and shared by the taps it is in.
+struct SplitRow {
+    const float *a, *b, *s;   // halves and their sum across the block, at the thread's column
+    __device__ __forceinline__ float tap(int u, int l) const { return s[u] - a[l] - b[l]; }
+};
+__device__ __forceinline__ float dxForward(const Grid2D& g, const SplitRow& f) {
+    return weigh(g, f.tap(1, 0), f.tap(2, -1), f.tap(3, -2), f.tap(4, -3));
 }
-// Forward z derivative (rows i+1..i+4 minus i..i-3).
-__device__ __forceinline__ float dzForward(const Grid2D& g, const Split& f) {
-    return g.c1 * f.tap(1, 0, 0, 0) + g.c2 * f.tap(2, 0, -1, 0) + g.c3 * f.tap(3, 0, -2, 0) + g.c4 * f.tap(4, 0, -3, 0);
+__device__ __forceinline__ float dxBackward(const Grid2D& g, const SplitRow& f) {
+    return weigh(g, f.tap(0, -1), f.tap(1, -2), f.tap(2, -3), f.tap(3, -4));
 }
-// Backward z derivative (rows i..i+3 minus i-1..i-4).
-__device__ __forceinline__ float dzBackward(const Grid2D& g, const Split& f) {
-    return g.c1 * f.tap(0, 0, -1, 0) + g.c2 * f.tap(1, 0, -2, 0) + g.c3 * f.tap(2, 0, -3, 0) + g.c4 * f.tap(3, 0, -4, 0);
-}
+template <int R> struct SplitColumn {
+    Column<R> a, b;
+    float s[R + 7];
+    __device__ __forceinline__ void sum() {
+#pragma unroll
+        for (int k = 0; k < R + 7; ++k) s[k] = a.v[k] + b.v[k];
+    }
+    __device__ __forceinline__ float tap(int u, int l) const { return s[u] - a.v[l] - b.v[l]; }
+    // z derivative of own row r: 8 rows from r, both directions (the column starts 3 rows above the
+    // strip for the forward one, 4 for the backward one).
+    __device__ __forceinline__ float dz(const Grid2D& g, int r) const {
+        return weigh(g, tap(r + 4, r + 3), tap(r + 5, r + 2), tap(r + 6, r + 1), tap(r + 7, r));
+    }
+};
 
 // Total-field derivatives of the hybrid scheme (Cuda_Check.cu:324-334, 377-387).
-__device__ __forceinline__ float dxForward(const Grid2D& g, const TileRef& f) {
-    return g.c1 * (f(0, 1) - f(0, 0)) + g.c2 * (f(0, 2) - f(0, -1)) + g.c3 * (f(0, 3) - f(0, -2)) + g.c4 * (f(0, 4) - f(0, -3));
+__device__ __forceinline__ float dxForward(const Grid2D& g, const float* f) {
+    return weigh(g, f[1] - f[0], f[2] - f[-1], f[3] - f[-2], f[4] - f[-3]);
 }
-__device__ __forceinline__ float dxBackward(const Grid2D& g, const TileRef& f) {
-    return g.c1 * (f(0, 0) - f(0, -1)) + g.c2 * (f(0, 1) - f(0, -2)) + g.c3 * (f(0, 2) - f(0, -3)) + g.c4 * (f(0, 3) - f(0, -4));
+__device__ __forceinline__ float dxBackward(const Grid2D& g, const float* f) {
+    return weigh(g, f[0] - f[-1], f[1] - f[-2], f[2] - f[-3], f[3] - f[-4]);
 }
-__device__ __forceinline__ float dzForward(const Grid2D& g, const TileRef& f) {
-    return g.c1 * (f(1, 0) - f(0, 0)) + g.c2 * (f(2, 0) - f(-1, 0)) + g.c3 * (f(3, 0) - f(-2, 0)) + g.c4 * (f(4, 0) - f(-3, 0));
+template <int R> __device__ __forceinline__ float dzAt(const Grid2D& g, const Column<R>& c, int r) {
+    return weigh(g, c.v[r + 4] - c.v[r + 3], c.v[r + 5] - c.v[r + 2], c.v[r + 6] - c.v[r + 1], c.v[r + 7] - c.v[r]);
 }
-__device__ __forceinline__ float dzBackward(const Grid2D& g, const TileRef& f) {
-    return g.c1 * (f(0, 0) - f(-1, 0)) + g.c2 * (f(1, 0) - f(-2, 0)) + g.c3 * (f(2, 0) - f(-3, 0)) + g.c4 * (f(3, 0) - f(-4, 0));
+
+// The same with the term as it is.
+__device__ __forceinline__ float advanceBy(const Grid2D& g, float old, float d, float term) {
+    return __fmaf_rn(old, g.inv_dt - d, term) / (g.inv_dt + d);
+}
+
+// ---- cell updates --------------------------------------------------------------------------
+
+struct Damp { float x, xh, z, zh; };   // of one cell, whole and half node, along x and z
+
+template <int R> __device__ __forceinline__ Damp Damping<R>::at(int r, bool undamped) const {
+    return Damp{x, xh, undamped ? 0.0f : z[r], undamped ? 0.0f : zh[r]};
+}
+
+// Hybrid stresses (Cuda_Check.cu:315-364): totals inside, sums of damped halves in the layer.
+// h: sxz1, sxz2, sxx1, szz1, sxx2, szz2.
+__device__ __forceinline__ void hybridStress(const Grid2D& g, bool pml, const Damp& d, float muZ, float l2mX, float lambdaX,
+                                             float dvz_dx, float dvx_dz, float dvx_dx, float dvz_dz, float& sxz, float& sxx,
+                                             float& szz, float (&h)[6]) {
+    if (!pml) {
+        sxz = __fmaf_rn(g.dt * muZ, dvz_dx + dvx_dz, sxz);
+        sxx = __fmaf_rn(g.dt, __fmaf_rn(l2mX, dvx_dx, __fmul_rn(lambdaX, dvz_dz)), sxx);
+        szz = __fmaf_rn(g.dt, __fmaf_rn(lambdaX, dvx_dx, __fmul_rn(l2mX, dvz_dz)), szz);
+        return;
+    }
+    h[0] = advance(g, h[0], d.x, muZ, dvz_dx);
+    h[1] = advance(g, h[1], d.zh, muZ, dvx_dz);
+    h[2] = advance(g, h[2], d.xh, l2mX, dvx_dx);
+    h[3] = advance(g, h[3], d.xh, lambdaX, dvx_dx);
+    h[4] = advance(g, h[4], d.z, lambdaX, dvz_dz);
+    h[5] = advance(g, h[5], d.z, l2mX, dvz_dz);
+    sxz = h[0] + h[1];
+    sxx = h[2] + h[4];
+    szz = h[3] + h[5];
+}
+
+// Hybrid velocities (Cuda_Check.cu:368-412).  h: vz1, vz2, vx1, vx2.
+__device__ __forceinline__ void hybridVelocity(const Grid2D& g, bool pml, const Damp& d, float rhoXZ, float rho,
+                                               float dsigxz_dx, float dsigzz_dz, float dsigxx_dx, float dsigxz_dz, float& vx,
+                                               float& vz, float (&h)[4]) {
+    if (!pml) {
+        vz = __fmaf_rn(g.dt * (dsigxz_dx + dsigzz_dz), __fdividef(1.0f, rhoXZ), vz);
+        vx = __fmaf_rn(g.dt * (dsigxx_dx + dsigxz_dz), __fdividef(1.0f, rho), vx);
+        return;
+    }
+    h[0] = advanceBy(g, h[0], d.xh, dsigxz_dx / rhoXZ);
+    h[1] = advanceBy(g, h[1], d.zh, dsigzz_dz / rhoXZ);
+    h[2] = advanceBy(g, h[2], d.x, dsigxx_dx / rho);
+    h[3] = advanceBy(g, h[3], d.z, dsigxz_dz / rho);
+    vx = h[2] + h[3];
+    vz = h[0] + h[1];
+}
+
+// The stress-type point source, half of it into each split half.
+__device__ __forceinline__ void addSplitSource(const Control2D& c, float w, float (&s)[6]) {
+    const float half = w * 0.5f;
+    if (c.srcType == SEIS2D_EXPLOSIVE) {
+#pragma unroll
+        for (int h = 0; h < 4; ++h) s[h] = __fadd_rn(s[h], half);
+    } else {
+        s[4] = __fadd_rn(s[4], half); s[5] = __fadd_rn(s[5], half);
+    }
+}
+
+// Split-field stresses (Cuda_Check.cu:224-266, 453-487).  s: sxx1, sxx2, szz1, szz2, sxz1, sxz2.
+__device__ __forceinline__ void splitStress(const Grid2D& g, const Damp& d, float mu, float l2m, float lambda, float dvx_dx,
+                                            float dvz_dz, float dvz_dx, float dvx_dz, float (&s)[6]) {
+    s[0] = advance(g, s[0], d.xh, l2m, dvx_dx);
+    s[1] = advance(g, s[1], d.z, lambda, dvz_dz);
+    s[2] = advance(g, s[2], d.xh, lambda, dvx_dx);
+    s[3] = advance(g, s[3], d.z, l2m, dvz_dz);
+    s[4] = advance(g, s[4], d.x, mu, dvz_dx);
+    s[5] = advance(g, s[5], d.zh, mu, dvx_dz);
+}
+
+// The traction-free row (Cuda_Check.cu:431-452); the shear derivatives take two taps there.
+__device__ __forceinline__ void freeRowStress(const Grid2D& g, const Damp& d, float mu, float dp, float dvx_dx, float dvz_dx,
+                                              float dvx_dz, float (&s)[6]) {
+    s[0] = advance(g, s[0], d.xh, dp, dvx_dx);
+    s[1] = s[2] = s[3] = 0.0f;
+    s[4] = advance(g, s[4], d.x, mu, dvz_dx);
+    s[5] = advance(g, s[5], d.zh, mu, dvx_dz);
+}
+__device__ __forceinline__ float weigh2(const Grid2D& g, float t1, float t2) { return __fmaf_rn(g.c1, t1, __fmul_rn(g.c2, t2)); }
+
+// Split-field velocities (Cuda_Check.cu:270-311, 512-563).  v: vx1, vx2, vz1, vz2.
+__device__ __forceinline__ void splitVelocity(const Grid2D& g, const Damp& d, float rho, float rhoMean, float dsigxx_dx,
+                                              float dsigxz_dz, float dsigxz_dx, float dsigzz_dz, float (&v)[4]) {
+    v[0] = advanceBy(g, v[0], d.x, dsigxx_dx / rho);
+    v[1] = advanceBy(g, v[1], d.z, dsigxz_dz / rho);
+    v[2] = advanceBy(g, v[2], d.xh, dsigxz_dx / rhoMean);
+    v[3] = advanceBy(g, v[3], d.zh, dsigzz_dz / rhoMean);
+}
+
+// The hybrid scheme's absorbing cells, whose totals are the sums of their halves.
+__device__ __forceinline__ bool inPml(const Grid2D& g, int i, int j) {
+    return i < g.npml || i >= g.NZ - g.npml || j < g.npml || j >= g.NX - g.npml;
+}
+
+// Rows of shared memory a strip needs: the arrays with x derivatives (halves and sum).
+template <int S> constexpr int kSharedArrays = S == kHybrid ? 2 : 6;
+
+// R rows of one array at the thread's column (own values and materials).
+template <int R> __device__ __forceinline__ void loadRows(float (&v)[R], const float* f, const Grid2D& g, int row, int j) {
+#pragma unroll
+    for (int r = 0; r < R; ++r) v[r] = row + r < g.NZ ? __ldcg(f + (row + r) * g.NX + j) : 0.0f;
 }
 
 // Receiver sample of the current state (extractReceiverSamplesKernel, Cuda_Check.cu:793-818).
@@ -182,137 +328,166 @@ __device__ __forceinline__ bool stressSource(const Control2D& c, int step, float
 
 // ---- stress ----------------------------------------------------------------------------
 
-// Split-field stress update of Types 1 and 3 (Cuda_Check.cu:224-266, 416-487) with the
-// free-surface mirror of :491-508 written by the owners of the mirrored rows.
-// Stress update of tile (bx, by) at `step`; `pendingOk` allows folding in the stress-type
-// source of step-1 (false for the first step of a batch, whose source the batch end applied).
-// All threads of the block call it; `tiles` holds 4 tiles of shared memory.
-template <int S>
-__device__ __forceinline__ void stressTile(const Grid2D& g, const Fields2D& f, const Control2D& c, int step,
-                                           bool pendingOk, int bx, int by, float* tiles) {
-    const int i0 = by * kBY, j0 = bx * kBX;
+// Stress update of strip (bx, by) at `step`, all three schemes (Cuda_Check.cu:224-266, 315-364,
+// 416-487) with the free-surface mirror of :491-508 written by the owners of the mirrored rows;
+// `pendingOk` allows folding in the stress-type source of step-1 (false for the first step of
+// a batch, whose source the batch end applied).  All threads of the block call it.
+template <int S, int R>
+__device__ __forceinline__ void stressStrip(const Grid2D& g, const Fields2D& f, const Control2D& c, int step, bool pendingOk,
+                                            int bx, int by, Shared* sh) {
+    const int tid = threadIdx.x, j = bx * kCols + tid;
+    const int row = (S == kFree ? g.fs : 4) + by * R;
+    const bool inside = j < g.NX;
+    const bool own = tid >= kHalo && tid < kThreads - kHalo && j < g.NX - 4;   // j >= 4 by tid >= kHalo
+
     if (S == kHybrid) {
-        const float* src[2] = {f.vx, f.vz};
-        loadTiles(g, i0, j0, tiles, src, 2);
-    } else {
-        const float* src[4] = {f.vx1, f.vx2, f.vz1, f.vz2};
-        loadTiles(g, i0, j0, tiles, src, 4);
+        // vx forward in x and z, vz backward in both.
+        Column<R> vx, vz;
+        float muZ[R], l2mX[R], lambdaX[R], sxz[R], sxx[R], szz[R], half[R][6];
+        Damping<R> d;
+        if (own) {
+            const float* const halves[6] = {f.sxz1, f.sxz2, f.sxx1, f.szz1, f.sxx2, f.szz2};
+            d.load(g, f, row, j);
+#pragma unroll
+            for (int r = 0; r < R; ++r)
+                if (inPml(g, row + r, j) && row + r < g.NZ)
+#pragma unroll
+                    for (int h = 0; h < 6; ++h) half[r][h] = __ldcg(halves[h] + (row + r) * g.NX + j);
+            vx.load(f.vx, g, row - 3, j);
+            vz.load(f.vz, g, row - 4, j);
+            loadRows(muZ, f.muZ, g, row, j);
+            loadRows(l2mX, f.l2mX, g, row, j);
+            loadRows(lambdaX, f.lambdaX, g, row, j);
+            loadRows(sxz, f.sxz, g, row, j);
+            loadRows(sxx, f.sxx, g, row, j);
+            loadRows(szz, f.szz, g, row, j);
+        } else if (inside) {
+            vx.loadOwn(f.vx, g, row, j, 3);
+            vz.loadOwn(f.vz, g, row, j, 4);
+        }
+        if (inside) {
+#pragma unroll
+            for (int r = 0; r < R; ++r) {
+                sh[2 * r][tid] = vx.v[r + 3];
+                sh[2 * r + 1][tid] = vz.v[r + 4];
+            }
+        }
+        __syncthreads();
+        if (!own) return;
+#pragma unroll
+        for (int r = 0; r < R; ++r) {
+            const int i = row + r;
+            if (i >= g.NZ - 4) break;
+            const int k = i * g.NX + j;
+            const float dvz_dx = dxBackward(g, &sh[2 * r + 1][tid]);
+            const float dvx_dz = dzAt(g, vx, r);
+            const float dvx_dx = dxForward(g, &sh[2 * r][tid]);
+            const float dvz_dz = dzAt(g, vz, r);
+            const bool pml = inPml(g, i, j);
+            float w = 0.0f;
+            if (!pml && pendingOk && k == c.srcIdx && stressSource(c, step - 1, w)) {
+                if (c.srcType == SEIS2D_EXPLOSIVE) { sxx[r] = __fadd_rn(sxx[r], w); szz[r] = __fadd_rn(szz[r], w); }
+                else sxz[r] = __fadd_rn(sxz[r], w);
+            }
+            hybridStress(g, pml, d.at(r, false), muZ[r], l2mX[r], lambdaX[r], dvz_dx, dvx_dz, dvx_dx, dvz_dz, sxz[r], sxx[r],
+                         szz[r], half[r]);
+            if (pml) {
+                f.sxz1[k] = half[r][0]; f.sxz2[k] = half[r][1]; f.sxx1[k] = half[r][2];
+                f.szz1[k] = half[r][3]; f.sxx2[k] = half[r][4]; f.szz2[k] = half[r][5];
+            }
+            f.sxz[k] = sxz[r]; f.sxx[k] = sxx[r]; f.szz[k] = szz[r];
+        }
+        return;
+    }
+
+    SplitColumn<R> vx, vz;
+    float t[R][6];   // sxx1, sxx2, szz1, szz2, sxz1, sxz2
+    float mu[R + 1], l2m[R], l2mRight[R], lambda[R], lambdaRight[R];
+    Damping<R> d;
+    if (own) {
+        d.load(g, f, row, j);
+        vx.a.load(f.vx1, g, row - 3, j);
+        vx.b.load(f.vx2, g, row - 3, j);
+        vz.a.load(f.vz1, g, row - 4, j);
+        vz.b.load(f.vz2, g, row - 4, j);
+        const float* const stresses[6] = {f.sxx1, f.sxx2, f.szz1, f.szz2, f.sxz1, f.sxz2};
+#pragma unroll
+        for (int r = 0; r < R; ++r)
+#pragma unroll
+            for (int h = 0; h < 6; ++h) t[r][h] = row + r < g.NZ ? __ldcg(stresses[h] + (row + r) * g.NX + j) : 0.0f;
+        loadRows(l2m, f.l2m, g, row, j);
+        loadRows(l2mRight, f.l2m, g, row, j + 1);
+        loadRows(lambda, f.lambda, g, row, j);
+        loadRows(lambdaRight, f.lambda, g, row, j + 1);
+#pragma unroll
+        for (int r = 0; r <= R; ++r) mu[r] = row + r < g.NZ ? __ldcg(f.mu + (row + r) * g.NX + j) : 0.0f;
+    } else if (inside) {
+        vx.a.loadOwn(f.vx1, g, row, j, 3);
+        vx.b.loadOwn(f.vx2, g, row, j, 3);
+        vz.a.loadOwn(f.vz1, g, row, j, 4);
+        vz.b.loadOwn(f.vz2, g, row, j, 4);
+    }
+    if (inside) {
+        vx.sum();
+        vz.sum();
+#pragma unroll
+        for (int r = 0; r < R; ++r) {
+            sh[6 * r][tid] = vx.a.v[r + 3]; sh[6 * r + 1][tid] = vx.b.v[r + 3]; sh[6 * r + 2][tid] = vx.s[r + 3];
+            sh[6 * r + 3][tid] = vz.a.v[r + 4]; sh[6 * r + 4][tid] = vz.b.v[r + 4]; sh[6 * r + 5][tid] = vz.s[r + 4];
+        }
     }
     __syncthreads();
-    const int i = i0 + threadIdx.y, j = j0 + threadIdx.x;
-    const int firstRow = S == kFree ? g.fs : 4;
-    if (i < firstRow || i >= g.NZ - 4 || j < 4 || j >= g.NX - 4) return;
-    const int k = i * g.NX + j;
-    const float inv_dt = g.inv_dt;
-    float w = 0.0f;
-    const bool pending = pendingOk && k == c.srcIdx && stressSource(c, step - 1, w);
-
-    if (S == kHybrid) {
-        const TileRef vx{reinterpret_cast<float(*)[kTW]>(tiles)};
-        const TileRef vz{reinterpret_cast<float(*)[kTW]>(tiles + kTile)};
-        const float dvz_dx = dxBackward(g, vz);
-        const float dvx_dz = dzForward(g, vx);
-        const float dvx_dx = dxForward(g, vx);
-        const float dvz_dz = dzBackward(g, vz);
-        const bool is_pml = (i < g.npml || i >= g.NZ - g.npml || j < g.npml || j >= g.NX - g.npml);
-        if (!is_pml) {
-            float sxz = f.sxz[k], sxx = f.sxx[k], szz = f.szz[k];
-            if (pending) {
-                if (c.srcType == SEIS2D_EXPLOSIVE) { sxx = __fadd_rn(sxx, w); szz = __fadd_rn(szz, w); }
-                else sxz = __fadd_rn(sxz, w);
+    if (!own) return;
+#pragma unroll
+    for (int r = 0; r < R; ++r) {
+        const int i = row + r;
+        if (i >= g.NZ - 4) break;
+        const int k = i * g.NX + j;
+        const SplitRow rvx{&sh[6 * r][tid], &sh[6 * r + 1][tid], &sh[6 * r + 2][tid]};
+        const SplitRow rvz{&sh[6 * r + 3][tid], &sh[6 * r + 4][tid], &sh[6 * r + 5][tid]};
+        const Damp damp = d.at(r, S == kFree && i <= g.fs + 5);
+        float w = 0.0f;
+        if (pendingOk && k == c.srcIdx && stressSource(c, step - 1, w)) addSplitSource(c, w, t[r]);
+        const float muAvg = 0.5f * (mu[r] + mu[r + 1]);
+        const float dvx_dx = dxForward(g, rvx);
+        if (S == kFree && r == 0 && i == g.fs) {
+            freeRowStress(g, damp, muAvg, f.dp[j], dvx_dx, weigh2(g, rvz.tap(0, -1), rvz.tap(1, -2)),
+                          weigh2(g, vx.tap(r + 4, r + 3), vx.tap(r + 5, r + 2)), t[r]);
+        } else {
+            splitStress(g, damp, muAvg, 0.5f * (l2m[r] + l2mRight[r]), 0.5f * (lambda[r] + lambdaRight[r]), dvx_dx, vz.dz(g, r),
+                        dxBackward(g, rvz), vx.dz(g, r), t[r]);
+        }
+        f.sxx1[k] = t[r][0]; f.sxx2[k] = t[r][1]; f.szz1[k] = t[r][2];
+        f.szz2[k] = t[r][3]; f.sxz1[k] = t[r][4]; f.sxz2[k] = t[r][5];
+        if (S == kFree) {
+            // Odd images above the free surface (Cuda_Check.cu:491-508): szz of row fs+l into
+            // row fs-l, sxz of row fs+l-1 into row fs-l, l = 1..4.
+            const int l = i - g.fs;
+            if (l >= 1 && l <= 4) {
+                const int above = (g.fs - l) * g.NX + j;
+                f.szz1[above] = -t[r][2]; f.szz2[above] = -t[r][3];
             }
-            f.sxz[k] = sxz + g.dt * f.muZ[k] * (dvz_dx + dvx_dz);
-            f.sxx[k] = sxx + g.dt * (f.l2mX[k] * dvx_dx + f.lambdaX[k] * dvz_dz);
-            f.szz[k] = szz + g.dt * (f.lambdaX[k] * dvx_dx + f.l2mX[k] * dvz_dz);
-        } else {
-            const float d_z_val = f.dz[i], d_z_half_val = f.dzh[i];
-            const float d_x_val = f.dx[j], d_x_half_val = f.dxh[j];
-            const float sxz1 = (f.sxz1[k] * (inv_dt - d_x_val) + f.muZ[k] * dvz_dx) / (inv_dt + d_x_val);
-            const float sxz2 = (f.sxz2[k] * (inv_dt - d_z_half_val) + f.muZ[k] * dvx_dz) / (inv_dt + d_z_half_val);
-            const float sxx1 = (f.sxx1[k] * (inv_dt - d_x_half_val) + f.l2mX[k] * dvx_dx) / (inv_dt + d_x_half_val);
-            const float szz1 = (f.szz1[k] * (inv_dt - d_x_half_val) + f.lambdaX[k] * dvx_dx) / (inv_dt + d_x_half_val);
-            const float sxx2 = (f.sxx2[k] * (inv_dt - d_z_val) + f.lambdaX[k] * dvz_dz) / (inv_dt + d_z_val);
-            const float szz2 = (f.szz2[k] * (inv_dt - d_z_val) + f.l2mX[k] * dvz_dz) / (inv_dt + d_z_val);
-            f.sxz1[k] = sxz1; f.sxz2[k] = sxz2; f.sxx1[k] = sxx1; f.szz1[k] = szz1; f.sxx2[k] = sxx2; f.szz2[k] = szz2;
-            f.sxz[k] = sxz1 + sxz2;
-            f.sxx[k] = sxx1 + sxx2;
-            f.szz[k] = szz1 + szz2;
-        }
-        return;
-    }
-
-    const Split vx{TileRef{reinterpret_cast<float(*)[kTW]>(tiles)}, TileRef{reinterpret_cast<float(*)[kTW]>(tiles + kTile)}};
-    const Split vz{TileRef{reinterpret_cast<float(*)[kTW]>(tiles + 2 * kTile)},
-                   TileRef{reinterpret_cast<float(*)[kTW]>(tiles + 3 * kTile)}};
-    float d_z = f.dz[i], d_z_h = f.dzh[i];
-    if (S == kFree && i <= g.fs + 5) { d_z = 0.0f; d_z_h = 0.0f; }
-    const float d_x = f.dx[j], d_x_h = f.dxh[j];
-    float sxx1 = f.sxx1[k], sxx2 = f.sxx2[k], szz1 = f.szz1[k], szz2 = f.szz2[k], sxz1 = f.sxz1[k], sxz2 = f.sxz2[k];
-    if (pending) {
-        const float half = w * 0.5f;
-        if (c.srcType == SEIS2D_EXPLOSIVE) {
-            sxx1 = __fadd_rn(sxx1, half); sxx2 = __fadd_rn(sxx2, half);
-            szz1 = __fadd_rn(szz1, half); szz2 = __fadd_rn(szz2, half);
-        } else {
-            sxz1 = __fadd_rn(sxz1, half); sxz2 = __fadd_rn(sxz2, half);
-        }
-    }
-    const float muAvg = 0.5f * (f.mu[k] + f.mu[k + g.NX]);
-    if (S == kFree && i == g.fs) {
-        // Traction-free row (Cuda_Check.cu:431-452).
-        const float dvx_dx = dxForward(g, vx);
-        sxx1 = (sxx1 * (inv_dt - d_x_h) + f.dp[j] * dvx_dx) / (inv_dt + d_x_h);
-        const float dvz_dx = g.c1 * vz.tap(0, 0, 0, -1) + g.c2 * vz.tap(0, 1, 0, -2);
-        const float dvx_dz = g.c1 * vx.tap(1, 0, 0, 0) + g.c2 * vx.tap(2, 0, -1, 0);
-        sxz1 = (sxz1 * (inv_dt - d_x) + muAvg * dvz_dx) / (inv_dt + d_x);
-        sxz2 = (sxz2 * (inv_dt - d_z_h) + muAvg * dvx_dz) / (inv_dt + d_z_h);
-        f.szz1[k] = 0.0f; f.szz2[k] = 0.0f;
-        f.sxx1[k] = sxx1; f.sxx2[k] = 0.0f;
-        f.sxz1[k] = sxz1; f.sxz2[k] = sxz2;
-        // Shear image one row up (mirror l = 1 of Cuda_Check.cu:502-505).
-        f.sxz1[k - g.NX] = -sxz1; f.sxz2[k - g.NX] = -sxz2;
-        return;
-    }
-    const float dvx_dx = dxForward(g, vx);
-    const float dvz_dz = dzBackward(g, vz);
-    const float l2mAvg = 0.5f * (f.l2m[k] + f.l2m[k + 1]);
-    const float lamAvg = 0.5f * (f.lambda[k] + f.lambda[k + 1]);
-    sxx1 = (sxx1 * (inv_dt - d_x_h) + l2mAvg * dvx_dx) / (inv_dt + d_x_h);
-    sxx2 = (sxx2 * (inv_dt - d_z) + lamAvg * dvz_dz) / (inv_dt + d_z);
-    szz1 = (szz1 * (inv_dt - d_x_h) + lamAvg * dvx_dx) / (inv_dt + d_x_h);
-    szz2 = (szz2 * (inv_dt - d_z) + l2mAvg * dvz_dz) / (inv_dt + d_z);
-    const float dvz_dx = dxBackward(g, vz);
-    const float dvx_dz = dzForward(g, vx);
-    sxz1 = (sxz1 * (inv_dt - d_x) + muAvg * dvz_dx) / (inv_dt + d_x);
-    sxz2 = (sxz2 * (inv_dt - d_z_h) + muAvg * dvx_dz) / (inv_dt + d_z_h);
-    f.sxx1[k] = sxx1; f.sxx2[k] = sxx2; f.szz1[k] = szz1; f.szz2[k] = szz2; f.sxz1[k] = sxz1; f.sxz2[k] = sxz2;
-    if (S == kFree) {
-        // Odd images above the free surface (Cuda_Check.cu:491-508): szz of row fs+l into
-        // row fs-l, sxz of row fs+l-1 into row fs-l, l = 1..4.
-        const int l = i - g.fs;
-        if (l <= 4) {
-            const int above = (g.fs - l) * g.NX + j;
-            f.szz1[above] = -szz1; f.szz2[above] = -szz2;
-        }
-        if (l <= 3) {
-            const int above = (g.fs - l - 1) * g.NX + j;
-            f.sxz1[above] = -sxz1; f.sxz2[above] = -sxz2;
+            if (l <= 3) {
+                const int above = (g.fs - l - 1) * g.NX + j;
+                f.sxz1[above] = -t[r][4]; f.sxz2[above] = -t[r][5];
+            }
         }
     }
 }
 
-template <int S>
+template <int S, int R>
 __global__ void __launch_bounds__(kThreads) stressStep(Grid2D g, Fields2D f, const Control2D* __restrict__ ctl, int slot) {
+    __shared__ Shared sh[kSharedArrays<S> * R];
+    waitForPrevious();
     const Control2D c = *ctl;
     const int step = c.base + slot;
     if (blockIdx.y == gridDim.y - 1) {
         // Receiver row: the velocities of step-1 are final while the stresses update.
-        if (slot > 0)
-            recordStep<S>(g, f, c, step - 1, blockIdx.x * kThreads + threadIdx.y * kBX + threadIdx.x, kThreads * gridDim.x);
+        if (slot > 0) recordStep<S>(g, f, c, step - 1, blockIdx.x * kThreads + threadIdx.x, kThreads * gridDim.x);
         return;
     }
-    __shared__ float tiles[4 * kTile];
-    stressTile<S>(g, f, c, step, slot > 0, blockIdx.x, blockIdx.y, tiles);
+    stressStrip<S, R>(g, f, c, step, slot > 0, blockIdx.x, blockIdx.y, sh);
+    launchDependents();
 }
 
 // ---- velocity --------------------------------------------------------------------------
@@ -347,91 +522,152 @@ __device__ __forceinline__ void forceSource(const Grid2D& g, const Fields2D& f, 
     }
 }
 
-// Velocity update of the three schemes (Cuda_Check.cu:270-311, 368-412, 512-563) with the
-// outer-ring clear of zeroBoundaryKernel (:643-667) done by the ring's owners.
-template <int S>
-__device__ __forceinline__ void velocityTile(const Grid2D& g, const Fields2D& f, const Control2D& c, int step, int bx,
-                                             int by, float* tiles) {
-    const int i0 = by * kBY, j0 = bx * kBX;
-    if (S == kHybrid) {
-        const float* src[3] = {f.sxx, f.szz, f.sxz};
-        loadTiles(g, i0, j0, tiles, src, 3);
-    } else {
-        const float* src[6] = {f.sxx1, f.sxx2, f.szz1, f.szz2, f.sxz1, f.sxz2};
-        loadTiles(g, i0, j0, tiles, src, 6);
-    }
-    __syncthreads();
-    const int i = i0 + threadIdx.y, j = j0 + threadIdx.x;
-    if (i >= g.NZ || j >= g.NX) return;
-    const int k = i * g.NX + j;
-    if (i == 0 || i == g.NZ - 1 || j == 0 || j == g.NX - 1) {
+// The outer ring of velocities that zeroBoundaryKernel clears (Cuda_Check.cu:643-667): the first and
+// last column along the strip's rows, and with the first and last strip the rows beyond them.
+template <int S, int R> __device__ __forceinline__ void clearRing(const Grid2D& g, const Fields2D& f, int row, int j, bool last) {
+    if (j >= g.NX) return;
+    auto clear = [&](int i) {
+        const int k = i * g.NX + j;
         if (S == kHybrid) { f.vx[k] = 0.0f; f.vz[k] = 0.0f; }
         else { f.vx1[k] = 0.0f; f.vx2[k] = 0.0f; f.vz1[k] = 0.0f; f.vz2[k] = 0.0f; }
-        return;
+    };
+    const bool edge = j == 0 || j == g.NX - 1;
+    const int from = row == 4 ? 0 : row, to = last ? g.NZ : row + R;
+    if (edge)
+        for (int i = from; i < to; ++i) clear(i);
+    else {
+        if (row == 4) clear(0);
+        if (last) clear(g.NZ - 1);
     }
-    if (i < 4 || i >= g.NZ - 4 || j < 4 || j >= g.NX - 4) return;
+}
+
+// Velocity update of strip (bx, by), all three schemes (Cuda_Check.cu:270-311, 368-412, 512-563);
+// rows start at 4, so that the free surface's air rows are cleared too.
+template <int S, int R>
+__device__ __forceinline__ void velocityStrip(const Grid2D& g, const Fields2D& f, const Control2D& c, int step, int bx, int by,
+                                              bool lastStrip, Shared* sh) {
+    const int tid = threadIdx.x, j = bx * kCols + tid;
+    const int row = 4 + by * R;
+    const bool inside = j < g.NX;
+    const bool own = tid >= kHalo && tid < kThreads - kHalo && j < g.NX - 4;
     const float inv_dt = g.inv_dt;
 
     if (S == kHybrid) {
-        const TileRef sxx{reinterpret_cast<float(*)[kTW]>(tiles)};
-        const TileRef szz{reinterpret_cast<float(*)[kTW]>(tiles + kTile)};
-        const TileRef sxz{reinterpret_cast<float(*)[kTW]>(tiles + 2 * kTile)};
-        const float dsigxz_dx = dxForward(g, sxz);
-        const float dsigzz_dz = dzForward(g, szz);
-        const float dsigxx_dx = dxBackward(g, sxx);
-        const float dsigxz_dz = dzBackward(g, sxz);
-        const bool is_pml = (i < g.npml || i >= g.NZ - g.npml || j < g.npml || j >= g.NX - g.npml);
-        float vxNew, vzNew;
-        if (!is_pml) {
-            vzNew = f.vz[k] + g.dt * (dsigxz_dx + dsigzz_dz) / f.rhoXZ[k];
-            vxNew = f.vx[k] + g.dt * (dsigxx_dx + dsigxz_dz) / f.rhoOrig[k];
-        } else {
-            const float d_z_val = f.dz[i], d_z_half_val = f.dzh[i];
-            const float d_x_val = f.dx[j], d_x_half_val = f.dxh[j];
-            const float vz1 = (f.vz1[k] * (inv_dt - d_x_half_val) + dsigxz_dx / f.rhoXZ[k]) / (inv_dt + d_x_half_val);
-            const float vz2 = (f.vz2[k] * (inv_dt - d_z_half_val) + dsigzz_dz / f.rhoXZ[k]) / (inv_dt + d_z_half_val);
-            const float vx1 = (f.vx1[k] * (inv_dt - d_x_val) + dsigxx_dx / f.rhoOrig[k]) / (inv_dt + d_x_val);
-            const float vx2 = (f.vx2[k] * (inv_dt - d_z_val) + dsigxz_dz / f.rhoOrig[k]) / (inv_dt + d_z_val);
-            f.vz1[k] = vz1; f.vz2[k] = vz2; f.vx1[k] = vx1; f.vx2[k] = vx2;
-            vxNew = vx1 + vx2;
-            vzNew = vz1 + vz2;
+        // sxx backward in x, szz forward in z, sxz forward in x and backward in z.
+        Column<R> szz, sxz;
+        float sxx[R], vx[R], vz[R], rhoXZ[R], rho[R], half[R][4];
+        Damping<R> d;
+        if (own) {
+            const float* const halves[4] = {f.vz1, f.vz2, f.vx1, f.vx2};
+            d.load(g, f, row, j);
+#pragma unroll
+            for (int r = 0; r < R; ++r)
+                if (inPml(g, row + r, j) && row + r < g.NZ)
+#pragma unroll
+                    for (int h = 0; h < 4; ++h) half[r][h] = __ldcg(halves[h] + (row + r) * g.NX + j);
+            szz.load(f.szz, g, row - 3, j);
+            sxz.load(f.sxz, g, row - 4, j);
+            loadRows(vx, f.vx, g, row, j);
+            loadRows(vz, f.vz, g, row, j);
+            loadRows(rhoXZ, f.rhoXZ, g, row, j);
+            loadRows(rho, f.rhoOrig, g, row, j);
+        } else if (inside) {
+            sxz.loadOwn(f.sxz, g, row, j, 4);
         }
-        forceSource<S>(g, f, c, step, k, vxNew, vzNew);
-        f.vx[k] = vxNew; f.vz[k] = vzNew;
+        if (inside) {
+            loadRows(sxx, f.sxx, g, row, j);
+#pragma unroll
+            for (int r = 0; r < R; ++r) {
+                sh[2 * r][tid] = sxx[r];
+                sh[2 * r + 1][tid] = sxz.v[r + 4];
+            }
+        }
+        __syncthreads();
+        clearRing<S, R>(g, f, row, j, lastStrip);
+        if (!own) return;
+#pragma unroll
+        for (int r = 0; r < R; ++r) {
+            const int i = row + r;
+            if (i >= g.NZ - 4) break;
+            const int k = i * g.NX + j;
+            const float dsigxz_dx = dxForward(g, &sh[2 * r + 1][tid]);
+            const float dsigzz_dz = dzAt(g, szz, r);
+            const float dsigxx_dx = dxBackward(g, &sh[2 * r][tid]);
+            const float dsigxz_dz = dzAt(g, sxz, r);
+            const bool pml = inPml(g, i, j);
+            hybridVelocity(g, pml, d.at(r, false), rhoXZ[r], rho[r], dsigxz_dx, dsigzz_dz, dsigxx_dx, dsigxz_dz, vx[r], vz[r],
+                           half[r]);
+            if (pml) { f.vz1[k] = half[r][0]; f.vz2[k] = half[r][1]; f.vx1[k] = half[r][2]; f.vx2[k] = half[r][3]; }
+            forceSource<S>(g, f, c, step, k, vx[r], vz[r]);
+            f.vx[k] = vx[r]; f.vz[k] = vz[r];
+        }
         return;
     }
 
-    if (S == kFree && i < g.fs) {
-        f.vx1[k] = 0.0f; f.vx2[k] = 0.0f; f.vz1[k] = 0.0f; f.vz2[k] = 0.0f;
-        return;
+    SplitColumn<R> szz, sxz;
+    float sxx1[R], sxx2[R], v[R][4];   // vx1, vx2, vz1, vz2
+    float rho[R + 1], rhoRight[R + 1];
+    Damping<R> d;
+    if (own) {
+        d.load(g, f, row, j);
+        szz.a.load(f.szz1, g, row - 3, j);
+        szz.b.load(f.szz2, g, row - 3, j);
+        sxz.a.load(f.sxz1, g, row - 4, j);
+        sxz.b.load(f.sxz2, g, row - 4, j);
+        const float* const velocities[4] = {f.vx1, f.vx2, f.vz1, f.vz2};
+#pragma unroll
+        for (int r = 0; r < R; ++r)
+#pragma unroll
+            for (int h = 0; h < 4; ++h) v[r][h] = row + r < g.NZ ? __ldcg(velocities[h] + (row + r) * g.NX + j) : 0.0f;
+#pragma unroll
+        for (int r = 0; r <= R; ++r) {
+            rho[r] = row + r < g.NZ ? __ldcg(f.rho + (row + r) * g.NX + j) : 1.0f;
+            rhoRight[r] = row + r < g.NZ ? __ldcg(f.rho + (row + r) * g.NX + j + 1) : 1.0f;
+        }
+    } else if (inside) {
+        sxz.a.loadOwn(f.sxz1, g, row, j, 4);
+        sxz.b.loadOwn(f.sxz2, g, row, j, 4);
     }
-    const Split sxx{TileRef{reinterpret_cast<float(*)[kTW]>(tiles)}, TileRef{reinterpret_cast<float(*)[kTW]>(tiles + kTile)}};
-    const Split szz{TileRef{reinterpret_cast<float(*)[kTW]>(tiles + 2 * kTile)},
-                    TileRef{reinterpret_cast<float(*)[kTW]>(tiles + 3 * kTile)}};
-    const Split sxz{TileRef{reinterpret_cast<float(*)[kTW]>(tiles + 4 * kTile)},
-                    TileRef{reinterpret_cast<float(*)[kTW]>(tiles + 5 * kTile)}};
-    float d_z = f.dz[i], d_z_h = f.dzh[i];
-    if (S == kFree && i <= g.fs + 5) { d_z = 0.0f; d_z_h = 0.0f; }
-    const float d_x = f.dx[j], d_x_h = f.dxh[j];
-    const float cur_rho = f.rho[k];
-    const float dsigxx_dx = dxBackward(g, sxx);
-    const float dsigxz_dz = dzBackward(g, sxz);
-    float vx1 = (f.vx1[k] * (inv_dt - d_x) + dsigxx_dx / cur_rho) / (inv_dt + d_x);
-    const float vx2 = (f.vx2[k] * (inv_dt - d_z) + dsigxz_dz / cur_rho) / (inv_dt + d_z);
-    const float dsigxz_dx = dxForward(g, sxz);
-    const float dsigzz_dz = dzForward(g, szz);
-    const float rho_avg = 0.25f * (f.rho[k] + f.rho[k + 1] + f.rho[k + g.NX] + f.rho[k + g.NX + 1]);
-    float vz1 = (f.vz1[k] * (inv_dt - d_x_h) + dsigxz_dx / rho_avg) / (inv_dt + d_x_h);
-    const float vz2 = (f.vz2[k] * (inv_dt - d_z_h) + dsigzz_dz / rho_avg) / (inv_dt + d_z_h);
-    forceSource<S>(g, f, c, step, k, vx1, vz1);
-    f.vx1[k] = vx1; f.vx2[k] = vx2; f.vz1[k] = vz1; f.vz2[k] = vz2;
+    if (inside) {
+        loadRows(sxx1, f.sxx1, g, row, j);
+        loadRows(sxx2, f.sxx2, g, row, j);
+        szz.sum();
+        sxz.sum();
+#pragma unroll
+        for (int r = 0; r < R; ++r) {
+            sh[6 * r][tid] = sxx1[r]; sh[6 * r + 1][tid] = sxx2[r]; sh[6 * r + 2][tid] = sxx1[r] + sxx2[r];
+            sh[6 * r + 3][tid] = sxz.a.v[r + 4]; sh[6 * r + 4][tid] = sxz.b.v[r + 4]; sh[6 * r + 5][tid] = sxz.s[r + 4];
+        }
+    }
+    __syncthreads();
+    clearRing<S, R>(g, f, row, j, lastStrip);
+    if (!own) return;
+#pragma unroll
+    for (int r = 0; r < R; ++r) {
+        const int i = row + r;
+        if (i >= g.NZ - 4) break;
+        const int k = i * g.NX + j;
+        if (S == kFree && i < g.fs) {
+            f.vx1[k] = 0.0f; f.vx2[k] = 0.0f; f.vz1[k] = 0.0f; f.vz2[k] = 0.0f;
+            continue;
+        }
+        const SplitRow rxx{&sh[6 * r][tid], &sh[6 * r + 1][tid], &sh[6 * r + 2][tid]};
+        const SplitRow rxz{&sh[6 * r + 3][tid], &sh[6 * r + 4][tid], &sh[6 * r + 5][tid]};
+        const float rhoMean = 0.25f * (rho[r] + rhoRight[r] + rho[r + 1] + rhoRight[r + 1]);
+        splitVelocity(g, d.at(r, S == kFree && i <= g.fs + 5), rho[r], rhoMean, dxBackward(g, rxx), sxz.dz(g, r),
+                      dxForward(g, rxz), szz.dz(g, r), v[r]);
+        forceSource<S>(g, f, c, step, k, v[r][0], v[r][2]);
+        f.vx1[k] = v[r][0]; f.vx2[k] = v[r][1]; f.vz1[k] = v[r][2]; f.vz2[k] = v[r][3];
+    }
 }
 
-template <int S>
+template <int S, int R>
 __global__ void __launch_bounds__(kThreads) velocityStep(Grid2D g, Fields2D f, const Control2D* __restrict__ ctl, int slot) {
+    __shared__ Shared sh[kSharedArrays<S> * R];
+    waitForPrevious();
     const Control2D c = *ctl;
-    __shared__ float tiles[6 * kTile];
-    velocityTile<S>(g, f, c, c.base + slot, blockIdx.x, blockIdx.y, tiles);
+    velocityStrip<S, R>(g, f, c, c.base + slot, blockIdx.x, blockIdx.y, blockIdx.y == gridDim.y - 1, sh);
+    launchDependents();
 }
 
 // ---- multi-source injection (injectMultipleSourcesKernel, Cuda_Check.cu:822-834) ---------
@@ -554,7 +790,7 @@ struct BarrierLimits {
 // which case every block leaves the run.
 __device__ __forceinline__ bool gridBarrier(GridSync* gs, unsigned epoch, const BarrierLimits& lim) {
     __syncthreads();
-    if (threadIdx.x == 0 && threadIdx.y == 0) {
+    if (threadIdx.x == 0) {
         __threadfence();
         if (epoch != 1 || int(blockIdx.x) != lim.withheldBlock) atomicAdd(&gs->arrived, 1u);
         const unsigned target = epoch * gridDim.x;
@@ -572,28 +808,36 @@ __device__ __forceinline__ bool gridBarrier(GridSync* gs, unsigned epoch, const 
     return *reinterpret_cast<volatile unsigned*>(&gs->failed) == 0;
 }
 
+// Strips of a grid: across, and down for the stresses and the velocities.
+__host__ __device__ __forceinline__ int stripsAcross(const Grid2D& g) { return (g.NX - 8 + kCols - 1) / kCols; }
+__host__ __device__ __forceinline__ int stressStrips(const Grid2D& g, int scheme, int rows) {
+    return (g.NZ - 4 - (scheme == kFree ? g.fs : 4) + rows - 1) / rows;
+}
+__host__ __device__ __forceinline__ int velocityStrips(const Grid2D& g, int rows) { return (g.NZ - 8 + rows - 1) / rows; }
+
 // `count` steps from ctl->base with every block resident: per step the stress phase over all
-// tiles, a grid barrier, the velocity phase, a grid barrier.  The receivers of step-1 are
+// strips, a grid barrier, the velocity phase, a grid barrier.  The receivers of step-1 are
 // sampled after the stress phase (velocities are final then) and the last step is completed
 // as at a batch end.  Single-source runs only; multi-source runs use the per-step kernels.
-template <int S>
-__global__ void __launch_bounds__(kThreads, 3) runSteps(Grid2D g, Fields2D f, Control2D* ctl, GridSync* gs, int count,
-                                                        BarrierLimits lim) {
-    __shared__ float tiles[6 * kTile];
+template <int S, int R>
+__global__ void __launch_bounds__(kThreads, 4) runSteps(Grid2D g, Fields2D f, Control2D* ctl, GridSync* gs, int count,
+                                                     BarrierLimits lim) {
+    __shared__ Shared sh[kSharedArrays<S> * R];
     const Control2D c = *ctl;
-    const int tilesX = (g.NX + kBX - 1) / kBX, tilesY = (g.NZ + kBY - 1) / kBY, nTiles = tilesX * tilesY;
-    const int gtid = blockIdx.x * kThreads + threadIdx.y * kBX + threadIdx.x, gthreads = gridDim.x * kThreads;
+    const int across = stripsAcross(g), down = velocityStrips(g, R);
+    const int stress = across * stressStrips(g, S, R), velocity = across * down;
+    const int gtid = blockIdx.x * kThreads + threadIdx.x, gthreads = gridDim.x * kThreads;
     unsigned epoch = 0;
     for (int q = 0; q < count; ++q) {
         const int step = c.base + q;
-        for (int t = blockIdx.x; t < nTiles; t += gridDim.x) {
-            stressTile<S>(g, f, c, step, q > 0, t % tilesX, t / tilesX, tiles);
+        for (int t = blockIdx.x; t < stress; t += gridDim.x) {
+            stressStrip<S, R>(g, f, c, step, q > 0, t % across, t / across, sh);
             __syncthreads();
         }
         if (q > 0) recordStep<S>(g, f, c, step - 1, gtid, gthreads);
         if (!gridBarrier(gs, ++epoch, lim)) return;
-        for (int t = blockIdx.x; t < nTiles; t += gridDim.x) {
-            velocityTile<S>(g, f, c, step, t % tilesX, t / tilesX, tiles);
+        for (int t = blockIdx.x; t < velocity; t += gridDim.x) {
+            velocityStrip<S, R>(g, f, c, step, t % across, t / across, t / across == down - 1, sh);
             __syncthreads();
         }
         if (!gridBarrier(gs, ++epoch, lim)) return;
