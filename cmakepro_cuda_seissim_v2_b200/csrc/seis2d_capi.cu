@@ -6,6 +6,7 @@
 // many steps are captured once per batch length into a CUDA graph and replayed.
 #include "../../include/seis2d_capi.h"
 #include "seis2d_kernels.cuh"
+#include "seis2d_resident.cuh"
 
 #include <cuda.h>
 
@@ -140,6 +141,15 @@ int kernelScheme(int flag, bool upFlag) {
 
 }  // namespace
 
+// Run mode of a session until seis2d_set_run_mode chooses one: a persistent run where the grid
+// fits on the chip (planResident) and the run has at least kResidentSteps steps, else graph
+// replay.  Every grid that fits takes fewer us per step so (seis2d_resident.cuh), but a run also
+// loads and stores the state and ends with a look at its status.  One run and a synchronise,
+// graph against persistent in us: 8 steps 123/134 (440x420, free surface), 105/100 (hybrid),
+// 77/76 (120x100, split); 16 steps 198/194, 170/156, 113/101; 2 steps 65/77, 62/72, 54/68.
+constexpr int kRunByRule = -1;
+constexpr int kResidentSteps = 16;
+
 struct seis2d_session {
     Grid2D g{};
     int flag = 1;
@@ -166,9 +176,11 @@ struct seis2d_session {
     int gatherReceivers = 0, gatherStart = 0, gatherStride = 1, gatherSamples = 0, gatherTaken = 0;
     bool gatherOn = false;
     std::map<std::pair<int, int>, cudaGraphExec_t> graphs;  // (batch, with multi-source) -> graph
-    GridSync* gridSync = nullptr;   // barrier state of the persistent runs
-    int persistentBlocks = 0;       // co-resident blocks of the persistent kernel (0: not usable)
-    int runMode = SEIS2D_RUN_GRAPH;
+    GridSync* gridSync = nullptr;   // failure state of the persistent runs
+    ResidentPlan resident{};        // tiles of the persistent runs (px = 0: the grid does not fit on the chip)
+    int residentRows = 0, residentThreads = 0;
+    std::size_t residentShared = 0;
+    int runMode = kRunByRule;
     bool persistentPending = false; // a persistent run has not been checked yet
     BarrierLimits barrier{kBarrierCycles, -1};   // seis2d_debug_barrier_wait
     uint64_t launches = 0;
@@ -209,11 +221,12 @@ struct seis2d_session {
         return d;
     }
     void sync() {
+        GridSync state{};
+        const bool check = persistentPending;
+        if (check) cudaCheck(cudaMemcpyAsync(&state, gridSync, sizeof(state), cudaMemcpyDeviceToHost, stream), "read run status");
         cudaCheck(cudaStreamSynchronize(stream), "cudaStreamSynchronize");
-        if (persistentPending) {
+        if (check) {
             persistentPending = false;
-            GridSync state{};
-            cudaCheck(cudaMemcpy(&state, gridSync, sizeof(state), cudaMemcpyDeviceToHost), "read run status");
             if (state.failed) throw RuntimeError("A persistent run gave up at a grid barrier; its results are invalid");
         }
     }
@@ -293,25 +306,76 @@ void enqueueBatch(seis2d_session* s, int batch, bool multi) {
     s->launches += uint64_t(batch) * (multi ? 3 : 2) + 1;
 }
 
-// Blocks of the persistent kernel that fit on the device at once (cooperative launch bound).
-template <int S, int R> int residentBlocks() {
-    int device = 0, sms = 0, perSm = 0;
-    cudaCheck(cudaGetDevice(&device), "device");
-    cudaCheck(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device), "SM count");
-    cudaCheck(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&perSm, runSteps<S, R>, kThreads, 0), "occupancy");
-    return perSm * sms;
+// fn with the session's scheme and the rows of its resident cells as constants.
+template <class F> void dispatchResident(const seis2d_session* s, F&& fn) {
+    dispatch(s->scheme, [&](auto scheme) {
+        if (s->residentRows == 1) fn(scheme, std::integral_constant<int, 1>{});
+        else if (s->residentRows == 2) fn(scheme, std::integral_constant<int, 2>{});
+        else fn(scheme, std::integral_constant<int, 3>{});
+    });
+}
+
+// Tiles of a persistent run: one per SM at most, fewest rows per thread first, then the shortest
+// halo.  A tile side is at least the halo, so that halos come from direct neighbours.  Three rows
+// per thread is where the split schemes' arrays fill an SM's shared memory: 512 threads, 148 SMs
+// and 227k cells at most (460x460).
+void planResident(seis2d_session* s, int sms, std::size_t sharedLimit) {
+    const Grid2D& g = s->g;
+    const int words = s->scheme == kHybrid ? 1 : 2, arrays = s->scheme == kHybrid ? int(kHybridArrays) : int(kSplitArrays);
+    for (int rows = 1; rows <= 3 && !s->resident.px; ++rows) {
+        int shortest = std::numeric_limits<int>::max();
+        for (int px = 1; px <= sms && g.NX / px >= kHalo; ++px) {
+            const int pz = std::min(sms / px, g.NZ / kHalo);
+            const int width = (g.NX + px - 1) / px, height = (g.NZ + pz - 1) / pz;
+            const int threads = (width * ((height + rows - 1) / rows) + 31) / 32 * 32;
+            if (px * pz < 2 || threads > kResidentThreads || width + height >= shortest) continue;
+            if (2 * kHalo * (width + height) * words > kHaloWords * threads) continue;
+            const std::size_t shared = std::size_t(arrays) * kArea * sizeof(float) + kResidentReceivers * sizeof(int2);
+            if (width > kTileWidth || height > tileHeight(rows) || shared > sharedLimit) continue;
+            shortest = width + height;
+            s->resident = ResidentPlan{px, pz, std::max(width, height), kHalo * std::max(width, height) * words, nullptr};
+            s->residentRows = rows;
+            s->residentThreads = threads;
+            s->residentShared = shared;
+        }
+    }
+}
+
+std::size_t mailBytes(const ResidentPlan& p) { return std::size_t(p.px) * p.pz * 8 * p.side * sizeof(uint4); }
+
+// The mailboxes of persistent runs, from the first one on: at initialisation a session without
+// long runs would pay for them (on a small grid they are most of its memory).  Where they cannot
+// be had, or not now (the stream is being captured), the steps are replayed from graphs.
+bool residentReady(seis2d_session* s) {
+    if (s->resident.mail || !s->resident.px) return s->resident.px > 0;
+    cudaStreamCaptureStatus capturing = cudaStreamCaptureStatusNone;
+    if (cudaStreamIsCapturing(s->stream, &capturing) != cudaSuccess || capturing != cudaStreamCaptureStatusNone) {
+        cudaGetLastError();
+        return false;
+    }
+    try {
+        dispatchResident(s, [&](auto tag, auto rows) {
+            cudaCheck(cudaFuncSetAttribute(residentRun<decltype(tag)::value, decltype(rows)::value>,
+                                           cudaFuncAttributeMaxDynamicSharedMemorySize, int(s->residentShared)),
+                      "persistent run shared memory");
+        });
+        s->resident.mail = reinterpret_cast<uint4*>(s->alloc<char>(mailBytes(s->resident)));
+    } catch (const std::exception&) {
+        cudaGetLastError();
+        s->resident.px = 0;
+        return false;
+    }
+    return true;
 }
 
 // One cooperative launch of `count` steps (after configure()).
 void launchPersistent(seis2d_session* s, int count) {
-    const int strips = stripsAcross(s->g) * velocityStrips(s->g, stripRows(s->g.total));
-    const int blocks = std::min(strips, s->persistentBlocks);
-    cudaCheck(cudaMemsetAsync(s->gridSync, 0, sizeof(GridSync), s->stream), "clear grid barrier");
-    dispatchStep(s, [&](auto tag, auto rows) {
+    dispatchResident(s, [&](auto tag, auto rows) {
         constexpr int S = decltype(tag)::value, R = decltype(rows)::value;
-        void* args[] = {&s->g, &s->f, &s->ctl, &s->gridSync, &count, &s->barrier};
-        cudaCheck(cudaLaunchCooperativeKernel(reinterpret_cast<void*>(runSteps<S, R>), dim3(blocks), dim3(kThreads), args, 0,
-                                              s->stream),
+        void* args[] = {&s->g, &s->f, &s->ctl, &s->gridSync, &count, &s->barrier, &s->resident};
+        cudaCheck(cudaLaunchCooperativeKernel(reinterpret_cast<void*>(residentRun<S, R>),
+                                              dim3(s->resident.px * s->resident.pz), dim3(s->residentThreads), args,
+                                              s->residentShared, s->stream),
                   "persistent launch");
     });
     s->launches += 1;
@@ -427,8 +491,9 @@ void noteGather(seis2d_session* s, int first, int count) {
     s->gatherTaken = int(std::max<int64_t>(s->gatherTaken, sample + 1));
 }
 
-void configure(seis2d_session* s, const Control2D& v) {
-    configureRun<<<1, 1, 0, s->stream>>>(s->ctl, v);
+// `exchanges`: those of the persistent run that follows (0: none does).
+void configure(seis2d_session* s, const Control2D& v, unsigned exchanges = 0) {
+    configureRun<<<1, 1, 0, s->stream>>>(s->ctl, v, s->gridSync, exchanges);
     cudaCheck(cudaGetLastError(), "configure run");
     s->launches += 1;
 }
@@ -676,6 +741,13 @@ int seis2d_initialize(seis2d_session** session, const seis2d_context* context) {
                 auto slot = [](std::size_t bytes) { return (std::max<std::size_t>(bytes, 16) + 255) & ~std::size_t(255); };
                 const std::size_t volumes = 14 + (c.flag_type == 2 ? 11 : 0);
                 const std::size_t lines = 4 + (c.flag_type == 3 ? 1 : 0);
+                int cooperative = 0, device = 0, sms = 0, shared = 0;
+                cudaCheck(cudaGetDevice(&device), "device");
+                cudaCheck(cudaDeviceGetAttribute(&cooperative, cudaDevAttrCooperativeLaunch, device), "cooperative launch");
+                cudaCheck(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device), "SM count");
+                cudaCheck(cudaDeviceGetAttribute(&shared, cudaDevAttrMaxSharedMemoryPerBlockOptin, device), "shared memory");
+                // The kernel's static shared memory (control block, counter) comes out of the same limit.
+                if (cooperative) planResident(s, sms, std::size_t(std::max(0, shared - 1024)));
                 s->arenaSize = volumes * slot(n * sizeof(float)) +
                                lines * slot(std::size_t(std::max(c.NX, c.NZ)) * sizeof(float)) +
                                slot(SEIS2D_MAX_ACTIVE_SOURCES * sizeof(seis2d_source)) + slot(sizeof(Control2D)) +
@@ -723,13 +795,6 @@ int seis2d_initialize(seis2d_session** session, const seis2d_context* context) {
             if (c.flag_type == 3) f.dp = s->upload(c.dp_flat.data, c.NX);
             s->ctl = s->carve<Control2D>(1);
             s->gridSync = s->carve<GridSync>(1);
-            int cooperative = 0, device = 0;
-            cudaCheck(cudaGetDevice(&device), "device");
-            cudaCheck(cudaDeviceGetAttribute(&cooperative, cudaDevAttrCooperativeLaunch, device), "cooperative launch");
-            if (cooperative)
-                dispatchStep(s, [&](auto tag, auto rows) {
-                    s->persistentBlocks = residentBlocks<decltype(tag)::value, decltype(rows)::value>();
-                });
             s->sync();
             *session = s;
             const int status = seis2d_update_receivers(s, c.rcv_grid_idx.data, c.num_rcv);
@@ -778,8 +843,12 @@ int seis2d_run_steps(seis2d_session* session, int first_it, int count, const sei
             throw InvalidArgument("Invalid GPU simulation state, iteration, or source count");
         if (count == 0) return;
         const bool multi = num_active_sources > 0;
-        configure(s, runControl(s, *context, first_it, num_active_sources, num_active_sources >= 0));
-        if (num_active_sources < 0 && s->runMode == SEIS2D_RUN_PERSISTENT && s->persistentBlocks > 0) {
+        const bool persistent = num_active_sources < 0 && !(s->gatherOn && s->gatherReceivers > kResidentReceivers) &&
+                                (s->runMode == SEIS2D_RUN_PERSISTENT || (s->runMode == kRunByRule && count >= kResidentSteps)) &&
+                                residentReady(s);
+        configure(s, runControl(s, *context, first_it, num_active_sources, num_active_sources >= 0),
+                  persistent ? 2u * unsigned(count) : 0u);
+        if (persistent) {
             launchPersistent(s, count);
             noteGather(s, first_it, count);
             return;

@@ -14,10 +14,12 @@
 //                  velocities is cleared by the threads that own it.
 //
 // plus, at the end of a batch, finishBatch (stress-type source and receivers of the last
-// step) so that the field state between API calls is the reference's.  Every tap is read
-// from a shared-memory tile that holds both split halves, so each expression keeps the
+// step) so that the field state between API calls is the reference's.  Threads own columns and
+// keep the rows around theirs in register windows (see "strips").  Each expression keeps the
 // reference's operand order ((a1 + a2 - b1 - b2) per tap, the same tap order and the same
 // averaging order) and the arithmetic matches the reference kernels operation for operation.
+// Grids that fit on the chip run many steps in one launch instead (seis2d_resident.cuh), with
+// the same cell updates and so the same bits.
 // The translation unit is compiled with --use_fast_math, the flag the reference builds its
 // 2-D solver with (CMakeLists.txt:128-135).
 //
@@ -104,8 +106,8 @@ template <int R> struct Column {
 #pragma unroll
         for (int k = 0; k < R + 7; ++k) {
             const int i = first + k;
-            // L2-only loads: in a persistent run other blocks rewrite these fields between the
-            // grid barriers, so neither the read-only path nor L1 may hold an old copy.
+            // L2-only loads: the next kernel rewrites these fields, and L1 keeps what is read again
+            // (materials, damping).
             v[k] = i < g.NZ ? __ldcg(f + i * g.NX + j) : 0.0f;
         }
     }
@@ -736,7 +738,20 @@ __global__ void injectSources(Grid2D g, Fields2D f, const Control2D* __restrict_
 
 // ---- batch boundaries ------------------------------------------------------------------
 
-__global__ void configureRun(Control2D* ctl, Control2D value) { *ctl = value; }
+// State of the persistent runs (seis2d_resident.cuh).
+struct GridSync {
+    unsigned failed;    // a wait of the last run gave up; its results are invalid
+    unsigned first;     // number of the exchange before the run's first
+    unsigned last;      // number of the run's last exchange
+    unsigned pad;
+};
+
+// Prepares the steps that follow in the stream.  A persistent run's exchanges are numbered here
+// and not by the host, so that a replay of a captured run has numbers of its own too.
+__global__ void configureRun(Control2D* ctl, Control2D value, GridSync* gs, unsigned exchanges) {
+    *ctl = value;
+    if (exchanges) *gs = GridSync{0, gs->last, gs->last + exchanges, 0};
+}
 
 // Completes the last step of a batch: its stress-type point source and its receivers, then
 // advances the clock by the batch length.
@@ -767,46 +782,19 @@ __global__ void finishBatch(Grid2D g, Fields2D f, Control2D* ctl, int slot, int 
     if (threadIdx.x == 0) ctl->base = c.base + batch;
 }
 
-// ---- persistent run (one cooperative launch for many steps) -----------------------------
+// ---- waits of a persistent run --------------------------------------------------------------
 
-// Grid barrier state of a persistent run, cleared before each launch.
-struct GridSync {
-    unsigned arrived;   // blocks that reached barriers so far (monotonic within a launch)
-    unsigned failed;    // a barrier wait gave up; the run's results are invalid
-    unsigned pad[2];
-};
-
-// Default bound of one barrier wait in SM clock cycles (about two seconds): the launch is
-// cooperative, so every block is resident and a normal wait ends in microseconds.
+// Default bound of one wait in SM clock cycles (about two seconds): the launch is cooperative,
+// so every block is resident and a normal wait ends in microseconds.
 constexpr long long kBarrierCycles = 4000000000LL;
 
-// Bound of the barrier waits and the withheld-arrival test hook of one persistent run.
+// Bound of the waits and the withheld-block test hook of one persistent run.
 struct BarrierLimits {
     long long cycles;     // bound of every wait
-    int withheldBlock;    // test hook: this block never arrives at the first barrier; -1 in use
+    int withheldBlock;    // test hook: this block sends nothing in its first exchange; -1 in use
 };
 
-// Grid-wide barrier number `epoch` (1, 2, ...): returns false when any wait timed out, in
-// which case every block leaves the run.
-__device__ __forceinline__ bool gridBarrier(GridSync* gs, unsigned epoch, const BarrierLimits& lim) {
-    __syncthreads();
-    if (threadIdx.x == 0) {
-        __threadfence();
-        if (epoch != 1 || int(blockIdx.x) != lim.withheldBlock) atomicAdd(&gs->arrived, 1u);
-        const unsigned target = epoch * gridDim.x;
-        const long long start = clock64();
-        while (*reinterpret_cast<volatile unsigned*>(&gs->arrived) < target) {
-            if (*reinterpret_cast<volatile unsigned*>(&gs->failed)) break;
-            if (clock64() - start > lim.cycles) {
-                atomicExch(&gs->failed, 1u);
-                break;
-            }
-        }
-        __threadfence();
-    }
-    __syncthreads();
-    return *reinterpret_cast<volatile unsigned*>(&gs->failed) == 0;
-}
+// ---- launch shapes -------------------------------------------------------------------------
 
 // Strips of a grid: across, and down for the stresses and the velocities.
 __host__ __device__ __forceinline__ int stripsAcross(const Grid2D& g) { return (g.NX - 8 + kCols - 1) / kCols; }
@@ -814,37 +802,6 @@ __host__ __device__ __forceinline__ int stressStrips(const Grid2D& g, int scheme
     return (g.NZ - 4 - (scheme == kFree ? g.fs : 4) + rows - 1) / rows;
 }
 __host__ __device__ __forceinline__ int velocityStrips(const Grid2D& g, int rows) { return (g.NZ - 8 + rows - 1) / rows; }
-
-// `count` steps from ctl->base with every block resident: per step the stress phase over all
-// strips, a grid barrier, the velocity phase, a grid barrier.  The receivers of step-1 are
-// sampled after the stress phase (velocities are final then) and the last step is completed
-// as at a batch end.  Single-source runs only; multi-source runs use the per-step kernels.
-template <int S, int R>
-__global__ void __launch_bounds__(kThreads, 4) runSteps(Grid2D g, Fields2D f, Control2D* ctl, GridSync* gs, int count,
-                                                     BarrierLimits lim) {
-    __shared__ Shared sh[kSharedArrays<S> * R];
-    const Control2D c = *ctl;
-    const int across = stripsAcross(g), down = velocityStrips(g, R);
-    const int stress = across * stressStrips(g, S, R), velocity = across * down;
-    const int gtid = blockIdx.x * kThreads + threadIdx.x, gthreads = gridDim.x * kThreads;
-    unsigned epoch = 0;
-    for (int q = 0; q < count; ++q) {
-        const int step = c.base + q;
-        for (int t = blockIdx.x; t < stress; t += gridDim.x) {
-            stressStrip<S, R>(g, f, c, step, q > 0, t % across, t / across, sh);
-            __syncthreads();
-        }
-        if (q > 0) recordStep<S>(g, f, c, step - 1, gtid, gthreads);
-        if (!gridBarrier(gs, ++epoch, lim)) return;
-        for (int t = blockIdx.x; t < velocity; t += gridDim.x) {
-            velocityStrip<S, R>(g, f, c, step, t % across, t / across, t / across == down - 1, sh);
-            __syncthreads();
-        }
-        if (!gridBarrier(gs, ++epoch, lim)) return;
-    }
-    finishStep<S>(g, f, c, c.base + count - 1, gtid, gthreads);
-    if (gtid == 0) ctl->base = c.base + count;
-}
 
 // recordReceiverStepOnGpu / copyReceiverRecordsFromGpu sample (Cuda_Check.cu:793-818).
 template <int S>

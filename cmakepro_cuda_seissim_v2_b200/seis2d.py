@@ -271,14 +271,15 @@ def runGpuSimulationStep(gpu: GPUSimData, current_it: int, ctx: SimulationContex
 
 def runGpuSimulationSteps(gpu: GPUSimData, first_it: int, count: int, ctx: SimulationContext,
                           num_active_sources: int = -1) -> None:
-    """``count`` steps from ``first_it`` replayed from a CUDA graph (equal to ``count`` calls of
-    runGpuSimulationStep; active sources advance like the reference time loop)."""
+    """``count`` steps from ``first_it`` in one persistent launch or replayed from a CUDA graph
+    (setRunMode; equal to ``count`` calls of runGpuSimulationStep; active sources advance like the reference time loop)."""
     c = ctx.to_c()
     _check(_lib().seis2d_run_steps(_session(gpu), int(first_it), int(count), byref(c), int(num_active_sources)))
 
 
 def setRunMode(gpu: GPUSimData, mode: int) -> None:
-    """capi2d.RUN_PERSISTENT (default) or capi2d.RUN_GRAPH for runGpuSimulationSteps."""
+    """capi2d.RUN_PERSISTENT or capi2d.RUN_GRAPH for runGpuSimulationSteps; until one is set,
+    runs of 16 steps or more on grids that fit on the chip are persistent."""
     _check(_lib().seis2d_set_run_mode(_session(gpu), int(mode)))
 
 

@@ -170,9 +170,8 @@ int seis2d_set_active_sources(seis2d_session* session, const seis2d_source* sour
 int seis2d_run_step(seis2d_session* session, int current_it, const seis2d_context* context,
                     int num_active_sources);
 /* count consecutive steps first_it .. first_it+count-1, equal to count calls of
- * seis2d_run_step, replayed from captured CUDA graphs of the per-step kernels (or, with
- * SEIS2D_RUN_PERSISTENT and a single source, one cooperative launch with two grid barriers
- * per step).  With num_active_sources >= 0 the active sources
+ * seis2d_run_step: with a single source and a grid that fits on the chip one cooperative launch
+ * (seis2d_run_mode), else replayed from captured CUDA graphs of the per-step kernels.  With num_active_sources >= 0 the active sources
  * advance by dt before each step and expire after 2.5 / f_peak, as the reference time loop
  * does on the host (src/Seis2D/Workflow2D.inc:300-318).  An open gather records the steps
  * it selects. */
@@ -216,10 +215,10 @@ int seis2d_synchronize(seis2d_session* session);
 /* Test hook (host-side fault injection): with nth > 0 the nth device allocation made by the
  * library from now on fails as out of memory, with the call's rollback; 0 disarms it. */
 void seis2d_debug_fail_allocation(int nth);
-/* Test hook of the bounded grid barriers of the persistent run mode (no reference
- * counterpart).  Every barrier wait gives up after `cycles` SM cycles (0 restores the default,
- * about two seconds), and with withheld_block >= 0 that block of the cooperative launch never
- * arrives at the first barrier, so every wait runs out: the blocks leave the run and the next
+/* Test hook of the bounded waits of persistent runs (no reference counterpart).  Every wait for
+ * another block gives up after `cycles` SM cycles (0 restores the default, about two seconds),
+ * and with withheld_block >= 0 that block of the cooperative launch sends nothing in its first
+ * exchange, so its neighbours' waits run out: the blocks leave the run and the next
  * synchronising call fails with SEIS2D_RUNTIME_ERROR.  -1 withholds nothing.  Meant for tests
  * of the failure path only. */
 int seis2d_debug_barrier_wait(seis2d_session* session, long long cycles, int withheld_block);
@@ -228,8 +227,11 @@ int seis2d_debug_barrier_wait(seis2d_session* session, long long cycles, int wit
  * caller are ordered after the steps as they are with the reference).  The session's own
  * non-blocking stream is the default; the previous stream is synchronised first. */
 int seis2d_set_stream(seis2d_session* session, void* stream);
-/* How seis2d_run_steps executes single-source runs (no reference counterpart); graph replay is
- * the default (on a B200 a grid barrier costs about as much as a kernel boundary). */
+/* How seis2d_run_steps executes single-source runs (no reference counterpart): one cooperative
+ * launch that keeps the state on the chip, or graph replay.  Until a mode is set, runs of at
+ * least 16 steps on a grid that fits on the chip (up to 227,000 cells on a B200) are persistent
+ * and all others replayed; a grid that does not fit is replayed in either mode.  The results are
+ * the same bits. */
 enum seis2d_run_mode { SEIS2D_RUN_PERSISTENT = 0, SEIS2D_RUN_GRAPH = 1 };
 int seis2d_set_run_mode(seis2d_session* session, int mode);
 /* Device time of count steps replayed as in seis2d_run_steps, split into the stress and
