@@ -475,9 +475,9 @@ PassKernel stressKernel(const seis3d_session* s) {
 }
 
 // Launch shapes of the two passes.
-struct Shape { dim3 grid, block; int zChunk; };
+struct Shape { dim3 grid, block; ZCuts cuts; };
 
-// Time of a pass over `planes` planes cut into chunks of c, in units of one plane of one CTA when
+// Time of a pass over `planes` planes cut into equal chunks of c (small grids and batches), in units of one plane of one CTA when
 // the device is full: what CTAs of `tiles` tiles cost on `slots` resident places.
 //   * Up to one CTA per SM (half the places) a CTA has its SM to itself: 0.7 of the full time per
 //     plane, and 2 planes' worth of start (rings, first stages, launch).  With the second CTA of
@@ -488,10 +488,9 @@ struct Shape { dim3 grid, block; int zChunk; };
 //     batch, where other shots fill it (three windows of 161x120x171 to 205x97x160: 649 us a
 //     step with 20-plane chunks, 681 with 8).
 // Fitted to the step times of 16 grids from 40x32x36 to 300x300x400 with chunks of 2 to 24
-// planes; the chunk it picks is within 1.7 % of the best one on average (5.6 % at most).  The
-// former rule (18 to 32 planes, whole rounds of places) left small grids to a few SMs:
-// 40x32x36 85.7 us a step against 24.1, 97x61x83 between walls 68.1 against 25.7, 161x120x171
-// with 20-cell CPML 260.8 against 229.2, 300x300x400 1334 against 1277.
+// planes; the chunk it picks is within 1.7 % of the best one on average (5.6 % at most).  Chunks
+// of 18 to 32 planes in whole rounds of places left small grids to a few SMs: 40x32x36 85.7 us a
+// step against 24.1, 97x61x83 between walls 68.1 against 25.7.
 double passTime(int tiles, int planes, int c, double slots, double tail) {
     const double rounds = tiles * double((planes + c - 1) / c) / slots;
     if (rounds <= 0.5) return 0.7 * (c + 2);
@@ -499,24 +498,57 @@ double passTime(int tiles, int planes, int c, double slots, double tail) {
     return (c + 0.8) * (rounds + tail * std::min(1.0, rounds - 1)) + 1.2;
 }
 
+// Chunks of `chunk` planes, evened out.
+ZCuts evenCuts(int planes, int chunk) {
+    const int chunks = (planes + chunk - 1) / chunk, c = (planes + chunks - 1) / chunks;
+    return ZCuts{{0, 0}, {c, c, c}};
+}
+
+// Chunks in three falling sizes, for passes of `load` planes per resident place, kFallingLoad or
+// more.  CTAs start in the order of their chunks, so the big ones, whose starts (rings, first
+// stages) cost the least, take most of the work, and the small ones fill the places that become
+// free at different times: with equal chunks the device stood part empty at the end of each pass.
+// 20 planes at most (24 and 32 cost more in L2 misses than they save in starts); nine twentieths
+// of a chunk per place are left to the next size.  us per step, equal chunks of the fitted size
+// against this: 128x128x128 with a 16-cell layer 174/134, 100^3 72/63, 60x60x500 165/130,
+// 300x50x300 with 20 cells 334/307, 213x199x187 376/351, 300x300x400 1267/1243; on average of
+// 15 grids 1.3 % from the best of 72 such rules.  Below kFallingLoad a place has too few planes to
+// cut: 72x64x90 38.3/39.6, 97x61x83 between walls 26.0/27.2.
+constexpr double kFallingLoad = 8.0;
+ZCuts fallingCuts(int planes, double load) {
+    ZCuts cuts;
+    const int c = std::min(20, int(0.75 * load + 0.5)), next = std::max(2, int(c / 2.5 + 0.5));
+    const double left = 0.45 / load;   // of the planes, per plane of a chunk
+    cuts.planes[0] = c;
+    cuts.planes[1] = next;
+    cuts.planes[2] = std::max(2, int(next / 3.0 + 0.5));
+    cuts.count[0] = int(planes * (1.0 - left * c) / c);
+    cuts.count[1] = std::max(0, int((planes * (1.0 - left * next) - cuts.count[0] * c) / next));
+    return cuts;
+}
+
+int zChunks(const ZCuts& cuts, int planes) {
+    const int cut = cuts.count[0] * cuts.planes[0] + cuts.count[1] * cuts.planes[1];
+    return cuts.count[0] + cuts.count[1] + (planes - cut + cuts.planes[2] - 1) / cuts.planes[2];
+}
+
 // `concurrent` sessions of a batch step together, each with its share of the places.
 Shape passShape(const seis3d_session* s, int concurrent = 1) {
     const int nxA = s->ctx.gx3D - 8, nyA = s->ctx.gy3D - 8, nzA = s->ctx.gz3D - 8;
     const int tilesX = (nxA + kTX - 1) / kTX, tilesY = (nyA + kTY - 1) / kTY;
+    const double slots = double(std::max(1, s->residentCtas)) / concurrent;
     int chunk = s->zChunk;
-    if (chunk <= 0) {
-        const double slots = double(std::max(1, s->residentCtas)) / concurrent;
+    if (chunk <= 0 && (concurrent > 1 || tilesX * tilesY * nzA / slots < kFallingLoad)) {
         double best = std::numeric_limits<double>::max();
         for (int c = 2; c <= 24; ++c) {
             const double t = passTime(tilesX * tilesY, nzA, c, slots, concurrent > 1 ? 0.0 : 0.9);
             if (t < best - 1e-9) { best = t; chunk = c; }
         }
     }
-    const int chunks = (nzA + chunk - 1) / chunk;
     Shape sh;
-    sh.zChunk = (nzA + chunks - 1) / chunks;
+    sh.cuts = chunk > 0 ? evenCuts(nzA, chunk) : fallingCuts(nzA, tilesX * tilesY * nzA / slots);
     sh.block = dim3(kTX, kWarps);
-    sh.grid = dim3(tilesX, tilesY, (nzA + sh.zChunk - 1) / sh.zChunk);
+    sh.grid = dim3(tilesX, tilesY, zChunks(sh.cuts, nzA));
     return sh;
 }
 
@@ -596,7 +628,7 @@ void enqueueStep(seis3d_session* s, const SourceParams& S, int slot, bool tail, 
     const Shape sh = passShape(s, concurrent);
     if (!stream) stream = s->stream;
     float* gather = s->gatherActive ? s->gather : nullptr;
-    const StepParams Q{sh.zChunk, tail ? 0 : slot, s->recv, s->recvCount, tail ? nullptr : gather};
+    const StepParams Q{sh.cuts, tail ? 0 : slot, s->recv, s->recvCount, tail ? nullptr : gather};
     if (ev) cudaEventRecord(ev->start, stream);
     launchPass(velocityKernel(s), sh, kVelocitySmem, stream, !ev && !tail && slot > 0, G, F, S, Q, "velocity pass");
     ++s->launches;
@@ -664,7 +696,7 @@ void tuneZChunk(seis3d_session* s) {
             s->zChunk = z;
             const Shape sh = passShape(s);
             auto pair = [&] {
-                const StepParams Q{sh.zChunk, 0, nullptr, 0, nullptr};
+                const StepParams Q{sh.cuts, 0, nullptr, 0, nullptr};
                 launchPass(velocityKernel(s), sh, kVelocitySmem, s->stream, false, G, F, S, Q, "z chunk tuning");
                 launchPass(stressKernel(s), sh, kStressSmem, s->stream, true, G, F, S, Q, "z chunk tuning");
                 s->launches += 2;
@@ -1531,7 +1563,7 @@ int seis3d_get_z_chunk(seis3d_session* s, int* setting, int* planes) {
         requireSession(s);
         if (!setting || !planes) throw InvalidArgument("Seis3D: null output.");
         *setting = s->zChunk;
-        *planes = passShape(s).zChunk;
+        *planes = passShape(s).cuts.planes[0];
     });
 }
 

@@ -63,9 +63,15 @@ struct SourceParams {
     float direction[3];
 };
 
+// The z extent cut into the chunks of a pass's CTAs: `count[0]` chunks of `planes[0]` planes, then
+// `count[1]` of `planes[1]`, and the rest in chunks of `planes[2]`.
+struct ZCuts {
+    int count[2], planes[3];
+};
+
 // One step of a pass as its launch gives it.
 struct StepParams {
-    int zChunk;            // planes per CTA
+    ZCuts cuts;
     int slot;              // steps since the clock's: the step executed is clock->step + slot
     const int4* receivers; // grid coordinates; sampled by the stress pass when `gather` is set
     int receiverCount;
