@@ -270,9 +270,9 @@ struct seis3d_session {
     int smCount = 148;
     int residentCtas = 296;         // CTAs of one pass resident on the whole device
     uint64_t launches = 0;          // kernels enqueued (graph replays add their node count)
-    float* uploadHost[kUploadSlots] = {};        // pinned chunks of seis3d_upload_model
+    float* uploadHost = nullptr;                 // pinned slots of seis3d_upload_model, one allocation
+    std::size_t uploadCapacity = 0;              // its floats
     cudaEvent_t uploadDone[kUploadSlots] = {};
-    std::size_t uploadCapacity = 0;              // cells per pinned chunk
     float* uploadRaw = nullptr;                  // device staging of seis3d_upload_model (3 volumes, then a flag)
     std::size_t uploadRawCells = 0;
     uint64_t graphNodes = 0;
@@ -342,8 +342,7 @@ void releaseSession(seis3d_session* s) noexcept {
     cudaFree(s->netCorr);
     if (s->hostRecv) cudaFreeHost(s->hostRecv);
     if (s->stage) cudaFreeHost(s->stage);
-    for (float* h : s->uploadHost)
-        if (h) cudaFreeHost(h);
+    if (s->uploadHost) cudaFreeHost(s->uploadHost);
     cudaFree(s->uploadRaw);
     for (cudaEvent_t e : s->uploadDone)
         if (e) cudaEventDestroy(e);
@@ -1213,7 +1212,7 @@ struct Packers {
     const float* volume[3];
     std::size_t total, chunk;
     int shares;
-    float* const* slots;
+    float* pinned;
     int chunks = int((total + chunk - 1) / chunk);
     std::atomic<int> open{0};                 // chunks below this have their slot free
     std::vector<std::atomic<int>> packed = std::vector<std::atomic<int>>(std::size_t(chunks));
@@ -1240,11 +1239,12 @@ struct Packers {
         } catch (const std::system_error&) {   // the caller's thread takes the shares without a thread
         }
     }
+    float* slot(int k) const { return pinned + (k % kUploadSlots) * 3 * chunk; }
     std::size_t cells(int k) const { return std::min(chunk, total - std::size_t(k) * chunk); }
     void pack(int k, int w) {
         const std::size_t count = cells(k), begin = count * w / shares, end = count * (w + 1) / shares;
         for (int a = 0; a < 3; ++a)
-            std::memcpy(slots[k % kUploadSlots] + a * chunk + begin, volume[a] + k * chunk + begin, (end - begin) * sizeof(float));
+            std::memcpy(slot(k) + a * chunk + begin, volume[a] + k * chunk + begin, (end - begin) * sizeof(float));
         packed[k].fetch_add(1, std::memory_order_release);
     }
     // The caller's part of chunk k; returns when the chunk is complete.
@@ -1287,14 +1287,13 @@ int seis3d_upload_model(seis3d_session* s, const seis3d_context* c, const float*
             ~Staging() { cudaStreamSynchronize(stream); }   // no copy outlives the call
         } staging{s->stream};
         const std::size_t chunk = std::min(kUploadCells, total);
-        if (s->uploadCapacity < chunk) {
-            for (auto& h : s->uploadHost) {
-                if (h) cudaFreeHost(h);
-                h = nullptr;
-            }
+        const int slots = int(std::min<std::size_t>(kUploadSlots, (total + chunk - 1) / chunk));
+        if (s->uploadCapacity < slots * chunk * 3) {
+            if (s->uploadHost) cudaFreeHost(s->uploadHost);
+            s->uploadHost = nullptr;
             s->uploadCapacity = 0;
-            for (auto& h : s->uploadHost) cudaCheck(hostMalloc(&h, chunk * 3 * sizeof(float)), "pinned model staging");
-            s->uploadCapacity = chunk;
+            cudaCheck(hostMalloc(&s->uploadHost, slots * chunk * 3 * sizeof(float)), "pinned model staging");
+            s->uploadCapacity = slots * chunk * 3;
         }
         for (auto& e : s->uploadDone)
             if (!e) cudaCheck(cudaEventCreateWithFlags(&e, cudaEventDisableTiming), "model staging event");
@@ -1312,7 +1311,7 @@ int seis3d_upload_model(seis3d_session* s, const seis3d_context* c, const float*
             }
             packers.finish(k);
             for (int a = 0; a < 3; ++a)
-                cudaCheck(cudaMemcpyAsync(raw + a * total + k * chunk, s->uploadHost[slot] + a * chunk,
+                cudaCheck(cudaMemcpyAsync(raw + a * total + k * chunk, packers.slot(k) + a * chunk,
                                           packers.cells(k) * sizeof(float), cudaMemcpyHostToDevice, s->stream), "upload model chunk");
             cudaCheck(cudaEventRecord(s->uploadDone[slot], s->stream), "model staging event");
         }
