@@ -142,13 +142,15 @@ int kernelScheme(int flag, bool upFlag) {
 }  // namespace
 
 // Run mode of a session until seis2d_set_run_mode chooses one: a persistent run where the grid
-// fits on the chip (planResident) and the run has at least kResidentSteps steps, else graph
-// replay.  Every grid that fits takes fewer us per step so (seis2d_resident.cuh), but a run also
-// loads and stores the state and ends with a look at its status.  One run and a synchronise,
+// fits on the chip (planResident), its threads take at most two rows of the split schemes, and the
+// run has at least kResidentSteps steps, else graph replay.  With three rows of split cells the
+// two are even (us per step, replayed against persistent: 440x420 split 7.5/7.7, free surface
+// 7.9/8.1; 400x380 7.4/7.2, 7.7/7.8), with fewer, or hybrid cells, the persistent run is faster
+// (seis2d_resident.cuh).  But it also loads and stores the state and ends with a look at its status.  One run and a synchronise,
 // graph against persistent in us: 8 steps 123/134 (440x420, free surface), 105/100 (hybrid),
 // 77/76 (120x100, split); 16 steps 198/194, 170/156, 113/101; 2 steps 65/77, 62/72, 54/68.
 constexpr int kRunByRule = -1;
-constexpr int kResidentSteps = 16;
+constexpr int kResidentSteps = 16, kResidentInvestment = 512;
 
 struct seis2d_session {
     Grid2D g{};
@@ -181,6 +183,7 @@ struct seis2d_session {
     int residentRows = 0, residentThreads = 0;
     std::size_t residentShared = 0;
     int runMode = kRunByRule;
+    int64_t longSteps = 0;          // steps of the runs by rule that a persistent run would suit
     bool persistentPending = false; // a persistent run has not been checked yet
     BarrierLimits barrier{kBarrierCycles, -1};   // seis2d_debug_barrier_wait
     uint64_t launches = 0;
@@ -287,7 +290,7 @@ template <class F> void dispatchStep(const seis2d_session* s, F&& fn) {
         const int rows = stripRows(s->g.total);
         if (rows == 1) fn(scheme, std::integral_constant<int, 1>{});
         else if (rows == 2) fn(scheme, std::integral_constant<int, 2>{});
-        else fn(scheme, std::integral_constant<int, 3>{});
+        else fn(scheme, std::integral_constant<int, 4>{});
     });
 }
 
@@ -342,6 +345,14 @@ void planResident(seis2d_session* s, int sms, std::size_t sharedLimit) {
 }
 
 std::size_t mailBytes(const ResidentPlan& p) { return std::size_t(p.px) * p.pz * 8 * p.side * sizeof(uint4); }
+
+// Whether a run of `count` steps by rule is persistent (kRunByRule).  The mailboxes are taken when the
+// session's long runs have come to kResidentInvestment steps: allocating them takes about 0.4 ms.
+bool residentPays(seis2d_session* s, int count) {
+    if (count < kResidentSteps || (s->scheme != kHybrid && s->residentRows > 2)) return false;
+    s->longSteps = std::min<int64_t>(s->longSteps + count, kResidentInvestment);
+    return s->resident.mail || s->longSteps >= kResidentInvestment;
+}
 
 // The mailboxes of persistent runs, from the first one on: at initialisation a session without
 // long runs would pay for them (on a small grid they are most of its memory).  Where they cannot
@@ -844,7 +855,7 @@ int seis2d_run_steps(seis2d_session* session, int first_it, int count, const sei
         if (count == 0) return;
         const bool multi = num_active_sources > 0;
         const bool persistent = num_active_sources < 0 && !(s->gatherOn && s->gatherReceivers > kResidentReceivers) &&
-                                (s->runMode == SEIS2D_RUN_PERSISTENT || (s->runMode == kRunByRule && count >= kResidentSteps)) &&
+                                (s->runMode == SEIS2D_RUN_PERSISTENT || (s->runMode == kRunByRule && residentPays(s, count))) &&
                                 residentReady(s);
         configure(s, runControl(s, *context, first_it, num_active_sources, num_active_sources >= 0),
                   persistent ? 2u * unsigned(count) : 0u);

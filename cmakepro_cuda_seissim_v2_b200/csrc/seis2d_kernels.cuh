@@ -43,11 +43,12 @@ constexpr int kThreads = 128;         // columns a block loads, one per thread
 constexpr int kHalo = 4;              // stencil radius (kStencilRadius, SolverNumerics.h:9)
 constexpr int kCols = kThreads - 2 * kHalo;   // columns a block updates
 
-// Rows a thread updates, 1 to 3.  More rows mean fewer halo rows read per cell (R + 7 for R), fewer
-// rows more blocks and a shorter chain in each: us a step of 1 / 2 / 3 / 4 rows on 120x100 4.5 / 5.2
-// / 6.0 / 7.0, 250x300 7.2 / 7.0 / 7.4 / 8.9, 440x420 11.4 / 10.3 / 9.5 / 9.9, 1601x1203 88 /
-// 75 / 69 / 78 (split halves; the hybrid scheme has the same order).
-__host__ __device__ __forceinline__ int stripRows(int cells) { return cells <= 40000 ? 1 : cells <= 100000 ? 2 : 3; }
+// Rows a thread updates.  More rows mean fewer halo rows read per cell (R + 7 for R), fewer rows more
+// blocks and a shorter chain in each: us a step of 1 / 2 / 3 / 4 rows on 120x100 4.1 / 4.9 / 5.2 /
+// 5.8, 250x220 5.6 / 5.7 / 5.6 / 6.1, 250x300 6.1 / 5.8 / 6.0 / 6.3, 400x350 8.3 / 7.3 / 7.4 / 7.4,
+// 440x420 9.3 / 8.5 / 7.6 / 7.5, 1601x1203 78 / 67 / 63 / 60 (split halves), 250x300 5.5 / 5.3 / 5.7
+// / 6.2, 1601x1203 46 / 40 / 38 / 37 (hybrid).
+__host__ __device__ __forceinline__ int stripRows(int cells) { return cells <= 55000 ? 1 : cells <= 150000 ? 2 : 4; }
 
 // Scheme ids of the kernels (flag_type, with flag 3 and upFlag off run as flag 1;
 // Cuda_Check.cu:1038-1046).
@@ -99,22 +100,31 @@ struct Control2D {
 // share.  All loads (the cells' own values and materials too) are issued before the one
 // barrier, so a block waits for memory once.
 
-// One array of a strip as its thread holds it: rows first .. first + R + 6 of its column.
+// Offsets of rows row-4 .. row+R+3 of a thread's column, formed once for all arrays: with an index, a
+// test and a 64-bit address for each load they were a third of a strip's instructions.  Rows past
+// the grid, in its last strip, repeat the last one: only cells that are not updated read them.
+template <int R> struct Rows {
+    unsigned o[R + 8];
+    __device__ __forceinline__ Rows(const Grid2D& g, int row, int j) {
+#pragma unroll
+        for (int k = 0; k < R + 8; ++k) o[k] = unsigned(min(row - 4 + k, g.NZ - 1)) * unsigned(g.NX) + unsigned(j);
+    }
+    __device__ __forceinline__ unsigned own(int r) const { return o[4 + r]; }
+};
+
+// One array of a strip as its thread holds it: R + 7 rows of its column, from `before` rows above its own.
 template <int R> struct Column {
     float v[R + 7];
-    __device__ __forceinline__ void load(const float* f, const Grid2D& g, int first, int j) {
+    __device__ __forceinline__ void load(const float* f, const Rows<R>& rows, int before) {
+        // L2-only loads: the next kernel rewrites these fields, and L1 keeps what is read again
+        // (materials, damping).
 #pragma unroll
-        for (int k = 0; k < R + 7; ++k) {
-            const int i = first + k;
-            // L2-only loads: the next kernel rewrites these fields, and L1 keeps what is read again
-            // (materials, damping).
-            v[k] = i < g.NZ ? __ldcg(f + i * g.NX + j) : 0.0f;
-        }
+        for (int k = 0; k < R + 7; ++k) v[k] = __ldcg(f + rows.o[4 - before + k]);
     }
     // The thread's own rows only, where they stand in a column that starts `before` rows earlier.
-    __device__ __forceinline__ void loadOwn(const float* f, const Grid2D& g, int row, int j, int before) {
+    __device__ __forceinline__ void loadOwn(const float* f, const Rows<R>& rows, int before) {
 #pragma unroll
-        for (int r = 0; r < R; ++r) v[before + r] = row + r < g.NZ ? __ldcg(f + (row + r) * g.NX + j) : 0.0f;
+        for (int r = 0; r < R; ++r) v[before + r] = __ldcg(f + rows.own(r));
     }
 };
 
@@ -290,9 +300,9 @@ __device__ __forceinline__ bool inPml(const Grid2D& g, int i, int j) {
 template <int S> constexpr int kSharedArrays = S == kHybrid ? 2 : 6;
 
 // R rows of one array at the thread's column (own values and materials).
-template <int R> __device__ __forceinline__ void loadRows(float (&v)[R], const float* f, const Grid2D& g, int row, int j) {
+template <int R> __device__ __forceinline__ void loadRows(float (&v)[R], const float* f, const Rows<R>& rows) {
 #pragma unroll
-    for (int r = 0; r < R; ++r) v[r] = row + r < g.NZ ? __ldcg(f + (row + r) * g.NX + j) : 0.0f;
+    for (int r = 0; r < R; ++r) v[r] = __ldcg(f + rows.own(r));
 }
 
 // Receiver sample of the current state (extractReceiverSamplesKernel, Cuda_Check.cu:793-818).
@@ -330,6 +340,80 @@ __device__ __forceinline__ bool stressSource(const Control2D& c, int step, float
 
 // ---- stress ----------------------------------------------------------------------------
 
+// Whether a strip of R rows has cells in the hybrid scheme's layer.  Strips without them run a body
+// without its halves, damping and tests.  With the shared offsets (Rows), at three rows: 1601x1203
+// cells with a 30-cell layer 44.8 -> 38.5 us a step, where the instructions issued (270 a cell, 0.7
+// of the issue slots) were the bound; split halves there 71.1 -> 64.0 by the offsets alone.
+template <int R> __device__ __forceinline__ bool touchesLayer(const Grid2D& g, int row, int bx) {
+    const int first = bx * kCols + kHalo;
+    return inPml(g, row, first) || inPml(g, row + R - 1, min(first + kCols, g.NX) - 1);
+}
+
+template <int R, bool kLayer>
+__device__ __forceinline__ void hybridStressStrip(const Grid2D& g, const Fields2D& f, const Control2D& c, int step, bool pendingOk,
+                                                  int row, int j, Shared* sh) {
+    const int tid = threadIdx.x;
+    const bool inside = j < g.NX;
+    const bool own = tid >= kHalo && tid < kThreads - kHalo && j < g.NX - 4;
+    const Rows<R> rows(g, row, j);
+    // vx forward in x and z, vz backward in both.
+    Column<R> vx, vz;
+    float muZ[R], l2mX[R], lambdaX[R], sxz[R], sxx[R], szz[R], half[R][6];
+    Damping<R> d;
+    if (own) {
+        const float* const halves[6] = {f.sxz1, f.sxz2, f.sxx1, f.szz1, f.sxx2, f.szz2};
+        if (kLayer) d.load(g, f, row, j);
+#pragma unroll
+        for (int r = 0; r < R; ++r)
+            if (kLayer && inPml(g, row + r, j))
+#pragma unroll
+                for (int h = 0; h < 6; ++h) half[r][h] = __ldcg(halves[h] + rows.own(r));
+        vx.load(f.vx, rows, 3);
+        vz.load(f.vz, rows, 4);
+        loadRows(muZ, f.muZ, rows);
+        loadRows(l2mX, f.l2mX, rows);
+        loadRows(lambdaX, f.lambdaX, rows);
+        loadRows(sxz, f.sxz, rows);
+        loadRows(sxx, f.sxx, rows);
+        loadRows(szz, f.szz, rows);
+    } else if (inside) {
+        vx.loadOwn(f.vx, rows, 3);
+        vz.loadOwn(f.vz, rows, 4);
+    }
+    if (inside) {
+#pragma unroll
+        for (int r = 0; r < R; ++r) {
+            sh[2 * r][tid] = vx.v[r + 3];
+            sh[2 * r + 1][tid] = vz.v[r + 4];
+        }
+    }
+    __syncthreads();
+    if (!own) return;
+#pragma unroll
+    for (int r = 0; r < R; ++r) {
+        const int i = row + r;
+        if (i >= g.NZ - 4) break;
+        const unsigned k = rows.own(r);
+        const float dvz_dx = dxBackward(g, &sh[2 * r + 1][tid]);
+        const float dvx_dz = dzAt(g, vx, r);
+        const float dvx_dx = dxForward(g, &sh[2 * r][tid]);
+        const float dvz_dz = dzAt(g, vz, r);
+        const bool pml = kLayer && inPml(g, i, j);
+        float w = 0.0f;
+        if (!pml && pendingOk && int(k) == c.srcIdx && stressSource(c, step - 1, w)) {
+            if (c.srcType == SEIS2D_EXPLOSIVE) { sxx[r] = __fadd_rn(sxx[r], w); szz[r] = __fadd_rn(szz[r], w); }
+            else sxz[r] = __fadd_rn(sxz[r], w);
+        }
+        hybridStress(g, pml, d.at(r, false), muZ[r], l2mX[r], lambdaX[r], dvz_dx, dvx_dz, dvx_dx, dvz_dz, sxz[r], sxx[r],
+                     szz[r], half[r]);
+        if (pml) {
+            f.sxz1[k] = half[r][0]; f.sxz2[k] = half[r][1]; f.sxx1[k] = half[r][2];
+            f.szz1[k] = half[r][3]; f.sxx2[k] = half[r][4]; f.szz2[k] = half[r][5];
+        }
+        f.sxz[k] = sxz[r]; f.sxx[k] = sxx[r]; f.szz[k] = szz[r];
+    }
+}
+
 // Stress update of strip (bx, by) at `step`, all three schemes (Cuda_Check.cu:224-266, 315-364,
 // 416-487) with the free-surface mirror of :491-508 written by the owners of the mirrored rows;
 // `pendingOk` allows folding in the stress-type source of step-1 (false for the first step of
@@ -341,64 +425,11 @@ __device__ __forceinline__ void stressStrip(const Grid2D& g, const Fields2D& f, 
     const int row = (S == kFree ? g.fs : 4) + by * R;
     const bool inside = j < g.NX;
     const bool own = tid >= kHalo && tid < kThreads - kHalo && j < g.NX - 4;   // j >= 4 by tid >= kHalo
+    const Rows<R> rows(g, row, j);
 
-    if (S == kHybrid) {
-        // vx forward in x and z, vz backward in both.
-        Column<R> vx, vz;
-        float muZ[R], l2mX[R], lambdaX[R], sxz[R], sxx[R], szz[R], half[R][6];
-        Damping<R> d;
-        if (own) {
-            const float* const halves[6] = {f.sxz1, f.sxz2, f.sxx1, f.szz1, f.sxx2, f.szz2};
-            d.load(g, f, row, j);
-#pragma unroll
-            for (int r = 0; r < R; ++r)
-                if (inPml(g, row + r, j) && row + r < g.NZ)
-#pragma unroll
-                    for (int h = 0; h < 6; ++h) half[r][h] = __ldcg(halves[h] + (row + r) * g.NX + j);
-            vx.load(f.vx, g, row - 3, j);
-            vz.load(f.vz, g, row - 4, j);
-            loadRows(muZ, f.muZ, g, row, j);
-            loadRows(l2mX, f.l2mX, g, row, j);
-            loadRows(lambdaX, f.lambdaX, g, row, j);
-            loadRows(sxz, f.sxz, g, row, j);
-            loadRows(sxx, f.sxx, g, row, j);
-            loadRows(szz, f.szz, g, row, j);
-        } else if (inside) {
-            vx.loadOwn(f.vx, g, row, j, 3);
-            vz.loadOwn(f.vz, g, row, j, 4);
-        }
-        if (inside) {
-#pragma unroll
-            for (int r = 0; r < R; ++r) {
-                sh[2 * r][tid] = vx.v[r + 3];
-                sh[2 * r + 1][tid] = vz.v[r + 4];
-            }
-        }
-        __syncthreads();
-        if (!own) return;
-#pragma unroll
-        for (int r = 0; r < R; ++r) {
-            const int i = row + r;
-            if (i >= g.NZ - 4) break;
-            const int k = i * g.NX + j;
-            const float dvz_dx = dxBackward(g, &sh[2 * r + 1][tid]);
-            const float dvx_dz = dzAt(g, vx, r);
-            const float dvx_dx = dxForward(g, &sh[2 * r][tid]);
-            const float dvz_dz = dzAt(g, vz, r);
-            const bool pml = inPml(g, i, j);
-            float w = 0.0f;
-            if (!pml && pendingOk && k == c.srcIdx && stressSource(c, step - 1, w)) {
-                if (c.srcType == SEIS2D_EXPLOSIVE) { sxx[r] = __fadd_rn(sxx[r], w); szz[r] = __fadd_rn(szz[r], w); }
-                else sxz[r] = __fadd_rn(sxz[r], w);
-            }
-            hybridStress(g, pml, d.at(r, false), muZ[r], l2mX[r], lambdaX[r], dvz_dx, dvx_dz, dvx_dx, dvz_dz, sxz[r], sxx[r],
-                         szz[r], half[r]);
-            if (pml) {
-                f.sxz1[k] = half[r][0]; f.sxz2[k] = half[r][1]; f.sxx1[k] = half[r][2];
-                f.szz1[k] = half[r][3]; f.sxx2[k] = half[r][4]; f.szz2[k] = half[r][5];
-            }
-            f.sxz[k] = sxz[r]; f.sxx[k] = sxx[r]; f.szz[k] = szz[r];
-        }
+    if constexpr (S == kHybrid) {
+        if (touchesLayer<R>(g, row, bx)) hybridStressStrip<R, true>(g, f, c, step, pendingOk, row, j, sh);
+        else hybridStressStrip<R, false>(g, f, c, step, pendingOk, row, j, sh);
         return;
     }
 
@@ -408,26 +439,26 @@ __device__ __forceinline__ void stressStrip(const Grid2D& g, const Fields2D& f, 
     Damping<R> d;
     if (own) {
         d.load(g, f, row, j);
-        vx.a.load(f.vx1, g, row - 3, j);
-        vx.b.load(f.vx2, g, row - 3, j);
-        vz.a.load(f.vz1, g, row - 4, j);
-        vz.b.load(f.vz2, g, row - 4, j);
+        vx.a.load(f.vx1, rows, 3);
+        vx.b.load(f.vx2, rows, 3);
+        vz.a.load(f.vz1, rows, 4);
+        vz.b.load(f.vz2, rows, 4);
         const float* const stresses[6] = {f.sxx1, f.sxx2, f.szz1, f.szz2, f.sxz1, f.sxz2};
 #pragma unroll
         for (int r = 0; r < R; ++r)
 #pragma unroll
-            for (int h = 0; h < 6; ++h) t[r][h] = row + r < g.NZ ? __ldcg(stresses[h] + (row + r) * g.NX + j) : 0.0f;
-        loadRows(l2m, f.l2m, g, row, j);
-        loadRows(l2mRight, f.l2m, g, row, j + 1);
-        loadRows(lambda, f.lambda, g, row, j);
-        loadRows(lambdaRight, f.lambda, g, row, j + 1);
+            for (int h = 0; h < 6; ++h) t[r][h] = __ldcg(stresses[h] + rows.own(r));
+        loadRows(l2m, f.l2m, rows);
+        loadRows(l2mRight, f.l2m + 1, rows);
+        loadRows(lambda, f.lambda, rows);
+        loadRows(lambdaRight, f.lambda + 1, rows);
 #pragma unroll
-        for (int r = 0; r <= R; ++r) mu[r] = row + r < g.NZ ? __ldcg(f.mu + (row + r) * g.NX + j) : 0.0f;
+        for (int r = 0; r <= R; ++r) mu[r] = __ldcg(f.mu + rows.own(r));
     } else if (inside) {
-        vx.a.loadOwn(f.vx1, g, row, j, 3);
-        vx.b.loadOwn(f.vx2, g, row, j, 3);
-        vz.a.loadOwn(f.vz1, g, row, j, 4);
-        vz.b.loadOwn(f.vz2, g, row, j, 4);
+        vx.a.loadOwn(f.vx1, rows, 3);
+        vx.b.loadOwn(f.vx2, rows, 3);
+        vz.a.loadOwn(f.vz1, rows, 4);
+        vz.b.loadOwn(f.vz2, rows, 4);
     }
     if (inside) {
         vx.sum();
@@ -444,12 +475,12 @@ __device__ __forceinline__ void stressStrip(const Grid2D& g, const Fields2D& f, 
     for (int r = 0; r < R; ++r) {
         const int i = row + r;
         if (i >= g.NZ - 4) break;
-        const int k = i * g.NX + j;
+        const unsigned k = rows.own(r);
         const SplitRow rvx{&sh[6 * r][tid], &sh[6 * r + 1][tid], &sh[6 * r + 2][tid]};
         const SplitRow rvz{&sh[6 * r + 3][tid], &sh[6 * r + 4][tid], &sh[6 * r + 5][tid]};
         const Damp damp = d.at(r, S == kFree && i <= g.fs + 5);
         float w = 0.0f;
-        if (pendingOk && k == c.srcIdx && stressSource(c, step - 1, w)) addSplitSource(c, w, t[r]);
+        if (pendingOk && int(k) == c.srcIdx && stressSource(c, step - 1, w)) addSplitSource(c, w, t[r]);
         const float muAvg = 0.5f * (mu[r] + mu[r + 1]);
         const float dvx_dx = dxForward(g, rvx);
         if (S == kFree && r == 0 && i == g.fs) {
@@ -543,6 +574,63 @@ template <int S, int R> __device__ __forceinline__ void clearRing(const Grid2D& 
     }
 }
 
+template <int R, bool kLayer>
+__device__ __forceinline__ void hybridVelocityStrip(const Grid2D& g, const Fields2D& f, const Control2D& c, int step, int row,
+                                                    int j, bool lastStrip, Shared* sh) {
+    const int tid = threadIdx.x;
+    const bool inside = j < g.NX;
+    const bool own = tid >= kHalo && tid < kThreads - kHalo && j < g.NX - 4;
+    const Rows<R> rows(g, row, j);
+    // sxx backward in x, szz forward in z, sxz forward in x and backward in z.
+    Column<R> szz, sxz;
+    float sxx[R], vx[R], vz[R], rhoXZ[R], rho[R], half[R][4];
+    Damping<R> d;
+    if (own) {
+        const float* const halves[4] = {f.vz1, f.vz2, f.vx1, f.vx2};
+        if (kLayer) d.load(g, f, row, j);
+#pragma unroll
+        for (int r = 0; r < R; ++r)
+            if (kLayer && inPml(g, row + r, j))
+#pragma unroll
+                for (int h = 0; h < 4; ++h) half[r][h] = __ldcg(halves[h] + rows.own(r));
+        szz.load(f.szz, rows, 3);
+        sxz.load(f.sxz, rows, 4);
+        loadRows(vx, f.vx, rows);
+        loadRows(vz, f.vz, rows);
+        loadRows(rhoXZ, f.rhoXZ, rows);
+        loadRows(rho, f.rhoOrig, rows);
+    } else if (inside) {
+        sxz.loadOwn(f.sxz, rows, 4);
+    }
+    if (inside) {
+        loadRows(sxx, f.sxx, rows);
+#pragma unroll
+        for (int r = 0; r < R; ++r) {
+            sh[2 * r][tid] = sxx[r];
+            sh[2 * r + 1][tid] = sxz.v[r + 4];
+        }
+    }
+    __syncthreads();
+    clearRing<kHybrid, R>(g, f, row, j, lastStrip);
+    if (!own) return;
+#pragma unroll
+    for (int r = 0; r < R; ++r) {
+        const int i = row + r;
+        if (i >= g.NZ - 4) break;
+        const unsigned k = rows.own(r);
+        const float dsigxz_dx = dxForward(g, &sh[2 * r + 1][tid]);
+        const float dsigzz_dz = dzAt(g, szz, r);
+        const float dsigxx_dx = dxBackward(g, &sh[2 * r][tid]);
+        const float dsigxz_dz = dzAt(g, sxz, r);
+        const bool pml = kLayer && inPml(g, i, j);
+        hybridVelocity(g, pml, d.at(r, false), rhoXZ[r], rho[r], dsigxz_dx, dsigzz_dz, dsigxx_dx, dsigxz_dz, vx[r], vz[r],
+                       half[r]);
+        if (pml) { f.vz1[k] = half[r][0]; f.vz2[k] = half[r][1]; f.vx1[k] = half[r][2]; f.vx2[k] = half[r][3]; }
+        forceSource<kHybrid>(g, f, c, step, k, vx[r], vz[r]);
+        f.vx[k] = vx[r]; f.vz[k] = vz[r];
+    }
+}
+
 // Velocity update of strip (bx, by), all three schemes (Cuda_Check.cu:270-311, 368-412, 512-563);
 // rows start at 4, so that the free surface's air rows are cleared too.
 template <int S, int R>
@@ -552,57 +640,11 @@ __device__ __forceinline__ void velocityStrip(const Grid2D& g, const Fields2D& f
     const int row = 4 + by * R;
     const bool inside = j < g.NX;
     const bool own = tid >= kHalo && tid < kThreads - kHalo && j < g.NX - 4;
-    const float inv_dt = g.inv_dt;
+    const Rows<R> rows(g, row, j);
 
-    if (S == kHybrid) {
-        // sxx backward in x, szz forward in z, sxz forward in x and backward in z.
-        Column<R> szz, sxz;
-        float sxx[R], vx[R], vz[R], rhoXZ[R], rho[R], half[R][4];
-        Damping<R> d;
-        if (own) {
-            const float* const halves[4] = {f.vz1, f.vz2, f.vx1, f.vx2};
-            d.load(g, f, row, j);
-#pragma unroll
-            for (int r = 0; r < R; ++r)
-                if (inPml(g, row + r, j) && row + r < g.NZ)
-#pragma unroll
-                    for (int h = 0; h < 4; ++h) half[r][h] = __ldcg(halves[h] + (row + r) * g.NX + j);
-            szz.load(f.szz, g, row - 3, j);
-            sxz.load(f.sxz, g, row - 4, j);
-            loadRows(vx, f.vx, g, row, j);
-            loadRows(vz, f.vz, g, row, j);
-            loadRows(rhoXZ, f.rhoXZ, g, row, j);
-            loadRows(rho, f.rhoOrig, g, row, j);
-        } else if (inside) {
-            sxz.loadOwn(f.sxz, g, row, j, 4);
-        }
-        if (inside) {
-            loadRows(sxx, f.sxx, g, row, j);
-#pragma unroll
-            for (int r = 0; r < R; ++r) {
-                sh[2 * r][tid] = sxx[r];
-                sh[2 * r + 1][tid] = sxz.v[r + 4];
-            }
-        }
-        __syncthreads();
-        clearRing<S, R>(g, f, row, j, lastStrip);
-        if (!own) return;
-#pragma unroll
-        for (int r = 0; r < R; ++r) {
-            const int i = row + r;
-            if (i >= g.NZ - 4) break;
-            const int k = i * g.NX + j;
-            const float dsigxz_dx = dxForward(g, &sh[2 * r + 1][tid]);
-            const float dsigzz_dz = dzAt(g, szz, r);
-            const float dsigxx_dx = dxBackward(g, &sh[2 * r][tid]);
-            const float dsigxz_dz = dzAt(g, sxz, r);
-            const bool pml = inPml(g, i, j);
-            hybridVelocity(g, pml, d.at(r, false), rhoXZ[r], rho[r], dsigxz_dx, dsigzz_dz, dsigxx_dx, dsigxz_dz, vx[r], vz[r],
-                           half[r]);
-            if (pml) { f.vz1[k] = half[r][0]; f.vz2[k] = half[r][1]; f.vx1[k] = half[r][2]; f.vx2[k] = half[r][3]; }
-            forceSource<S>(g, f, c, step, k, vx[r], vz[r]);
-            f.vx[k] = vx[r]; f.vz[k] = vz[r];
-        }
+    if constexpr (S == kHybrid) {
+        if (touchesLayer<R>(g, row, bx)) hybridVelocityStrip<R, true>(g, f, c, step, row, j, lastStrip, sh);
+        else hybridVelocityStrip<R, false>(g, f, c, step, row, j, lastStrip, sh);
         return;
     }
 
@@ -612,27 +654,27 @@ __device__ __forceinline__ void velocityStrip(const Grid2D& g, const Fields2D& f
     Damping<R> d;
     if (own) {
         d.load(g, f, row, j);
-        szz.a.load(f.szz1, g, row - 3, j);
-        szz.b.load(f.szz2, g, row - 3, j);
-        sxz.a.load(f.sxz1, g, row - 4, j);
-        sxz.b.load(f.sxz2, g, row - 4, j);
+        szz.a.load(f.szz1, rows, 3);
+        szz.b.load(f.szz2, rows, 3);
+        sxz.a.load(f.sxz1, rows, 4);
+        sxz.b.load(f.sxz2, rows, 4);
         const float* const velocities[4] = {f.vx1, f.vx2, f.vz1, f.vz2};
 #pragma unroll
         for (int r = 0; r < R; ++r)
 #pragma unroll
-            for (int h = 0; h < 4; ++h) v[r][h] = row + r < g.NZ ? __ldcg(velocities[h] + (row + r) * g.NX + j) : 0.0f;
+            for (int h = 0; h < 4; ++h) v[r][h] = __ldcg(velocities[h] + rows.own(r));
 #pragma unroll
         for (int r = 0; r <= R; ++r) {
-            rho[r] = row + r < g.NZ ? __ldcg(f.rho + (row + r) * g.NX + j) : 1.0f;
-            rhoRight[r] = row + r < g.NZ ? __ldcg(f.rho + (row + r) * g.NX + j + 1) : 1.0f;
+            rho[r] = __ldcg(f.rho + rows.own(r));
+            rhoRight[r] = __ldcg(f.rho + 1 + rows.own(r));
         }
     } else if (inside) {
-        sxz.a.loadOwn(f.sxz1, g, row, j, 4);
-        sxz.b.loadOwn(f.sxz2, g, row, j, 4);
+        sxz.a.loadOwn(f.sxz1, rows, 4);
+        sxz.b.loadOwn(f.sxz2, rows, 4);
     }
     if (inside) {
-        loadRows(sxx1, f.sxx1, g, row, j);
-        loadRows(sxx2, f.sxx2, g, row, j);
+        loadRows(sxx1, f.sxx1, rows);
+        loadRows(sxx2, f.sxx2, rows);
         szz.sum();
         sxz.sum();
 #pragma unroll
@@ -648,7 +690,7 @@ __device__ __forceinline__ void velocityStrip(const Grid2D& g, const Fields2D& f
     for (int r = 0; r < R; ++r) {
         const int i = row + r;
         if (i >= g.NZ - 4) break;
-        const int k = i * g.NX + j;
+        const unsigned k = rows.own(r);
         if (S == kFree && i < g.fs) {
             f.vx1[k] = 0.0f; f.vx2[k] = 0.0f; f.vz1[k] = 0.0f; f.vz2[k] = 0.0f;
             continue;

@@ -14,10 +14,10 @@
 // What bounds it: with one row per thread the exchange (a store, its visibility in L2 and the
 // load that sees it, twice a step: about 2.5 of 3.1 us), with three rows the instructions of the
 // cells, about 0.4 us per row and phase in hybrid cells and twice that in split ones.  us per
-// step, graph replay of the step kernels against this: split 120x100 4.4/3.2, 350x300 7.1/5.9,
-// 440x420 9.1/7.7; free surface 97x93 4.1/3.3, 250x300 6.5/5.0, 440x420 9.3/8.1; hybrid
-// 128x250 4.6/2.7, 250x300 6.2/3.9, 440x420 7.8/5.8.  Two grid barriers per step and the state
-// in L2 took 6.4 to 21 us.
+// step, graph replay of the step kernels against this: split 120x100 4.1/3.1, 300x240 5.8/5.2,
+// 440x420 7.5/7.7; free surface 97x93 3.9/3.2, 250x300 6.0/5.1, 440x420 7.9/8.1; hybrid 128x250
+// 3.9/2.7, 250x300 5.2/3.9, 440x420 7.4/6.0.  Two grid barriers per step and the state in L2 took
+// 6.4 to 21 us.
 //
 // All waits are bounded (BarrierLimits): a CTA that gives up sets the failure flag, which the
 // others see in their own waits, and every CTA leaves the run.

@@ -278,8 +278,8 @@ def runGpuSimulationSteps(gpu: GPUSimData, first_it: int, count: int, ctx: Simul
 
 
 def setRunMode(gpu: GPUSimData, mode: int) -> None:
-    """capi2d.RUN_PERSISTENT or capi2d.RUN_GRAPH for runGpuSimulationSteps; until one is set,
-    runs of 16 steps or more on grids that fit on the chip are persistent."""
+    """capi2d.RUN_PERSISTENT or capi2d.RUN_GRAPH for runGpuSimulationSteps; until one is set
+    the library chooses (long runs on grids that fit on the chip are persistent)."""
     _check(_lib().seis2d_set_run_mode(_session(gpu), int(mode)))
 
 

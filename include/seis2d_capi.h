@@ -228,9 +228,10 @@ int seis2d_debug_barrier_wait(seis2d_session* session, long long cycles, int wit
  * non-blocking stream is the default; the previous stream is synchronised first. */
 int seis2d_set_stream(seis2d_session* session, void* stream);
 /* How seis2d_run_steps executes single-source runs (no reference counterpart): one cooperative
- * launch that keeps the state on the chip, or graph replay.  Until a mode is set, runs of at
- * least 16 steps on a grid that fits on the chip (up to 227,000 cells on a B200) are persistent
- * and all others replayed; a grid that does not fit is replayed in either mode.  The results are
+ * launch that keeps the state on the chip, or graph replay.  Until a mode is set the library
+ * chooses: long runs (16 steps or more, once a session has made 512 of them) on grids that fit
+ * on the chip (on a B200 up to 227,000 cells in the hybrid scheme, 151,000 in the others) are
+ * persistent.  A grid of more than 227,000 cells is replayed in either mode.  The results are
  * the same bits. */
 enum seis2d_run_mode { SEIS2D_RUN_PERSISTENT = 0, SEIS2D_RUN_GRAPH = 1 };
 int seis2d_set_run_mode(seis2d_session* session, int mode);
