@@ -11,9 +11,9 @@
 // word is rewritten only after its reader has sent the words that the writer waited for in
 // between.
 //
-// What bounds it: with one row per thread the exchange (a store, its visibility in L2 and the
-// load that sees it, twice a step: about 2.5 of 3.1 us), with three rows the instructions of the
-// cells, about 0.4 us per row and phase in hybrid cells and twice that in split ones.  us per
+// What bounds it: with one row per thread mostly the exchange (a store, its visibility in L2 and the
+// load that sees it, twice a step), with more rows the instructions of the cells: hybrid tiles of
+// 1 / 2 / 3 rows take 2.7 / 3.9 / 5.9 us a step, split ones 3.1 / 6.0 / 7.7.  us per
 // step, graph replay of the step kernels against this: split 120x100 4.1/3.1, 300x240 5.8/5.2,
 // 440x420 7.5/7.7; free surface 97x93 3.9/3.2, 250x300 6.0/5.1, 440x420 7.9/8.1; hybrid 128x250
 // 3.9/2.7, 250x300 5.2/3.9, 440x420 7.4/6.0.  Two grid barriers per step and the state in L2 took
@@ -29,8 +29,8 @@ namespace seis2d {
 
 constexpr int kResidentThreads = 512;      // most threads of a tile
 // Shared-memory arrays of one fixed shape, so that a thread addresses its cells in all of them, and
-// the rows around them, by constant offsets from one register (with the shape in registers the
-// address arithmetic was half of a cell's instructions).
+// the rows around them, by constant offsets from one register (with the shape in registers a
+// cell took 807 instructions a step).
 constexpr int kPitch = 72, kTileWidth = kPitch - 2 * kHalo;       // floats per row
 constexpr int kTileRows = 55, kArea = kPitch * kTileRows + 8;     // floats per array
 __host__ __device__ constexpr int tileHeight(int rows) { return kTileRows - 2 * kHalo - rows; }   // windows reach past the tile

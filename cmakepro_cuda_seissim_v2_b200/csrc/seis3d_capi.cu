@@ -507,8 +507,8 @@ ZCuts evenCuts(int planes, int chunk) {
 // more.  CTAs start in the order of their chunks, so the big ones, whose starts (rings, first
 // stages) cost the least, take most of the work, and the small ones fill the places that become
 // free at different times: with equal chunks the device stood part empty at the end of each pass.
-// 20 planes at most (24 and 32 cost more in L2 misses than they save in starts); nine twentieths
-// of a chunk per place are left to the next size.  us per step, equal chunks of the fitted size
+// 20 planes at most (18, 22, 24 and 32 measured slower on average); nine twentieths of a chunk per
+// place are left to the next size.  us per step, equal chunks of the fitted size
 // against this: 128x128x128 with a 16-cell layer 174/134, 100^3 72/63, 60x60x500 165/130,
 // 300x50x300 with 20 cells 334/307, 213x199x187 376/351, 300x300x400 1267/1243; on average of
 // 15 grids 1.3 % from the best of 72 such rules.  Below kFallingLoad a place has too few planes to
@@ -1207,7 +1207,7 @@ int seis3d_upload_model_plane(seis3d_session* s, const seis3d_context* c, int z,
 
 // Host side of seis3d_upload_model: threads copy chunk after chunk of the three volumes into pinned
 // slots, each thread its share of every chunk, while the caller's thread hands full slots to the
-// copy engine.  The threads live for the call: started anew for each chunk they cost it 0.3 ms.
+// copy engine.  The threads live for the call, not for a chunk.
 struct Packers {
     const float* volume[3];
     std::size_t total, chunk;
