@@ -215,10 +215,13 @@ template <int S> struct HaloWords {
     }
 };
 
-// `count` steps from ctl->base; single-source runs only.
+// `count` steps from ctl->base; single-source runs only.  The control block is only read: the mailboxes
+// order neighbours, not a block that starts late against one that has finished, so a block that
+// moved `base` past the run could give a late one the wrong first step.  Every run has a
+// configureRun of its own, so nothing wants it moved.
 template <int S, int R>
-__global__ void __launch_bounds__(kResidentThreads, 1) residentRun(Grid2D g, Fields2D f, Control2D* ctl, GridSync* gs, int count,
-                                                                   BarrierLimits lim, ResidentPlan P) {
+__global__ void __launch_bounds__(kResidentThreads, 1) residentRun(Grid2D g, Fields2D f, const Control2D* ctl, GridSync* gs,
+                                                                   int count, BarrierLimits lim, ResidentPlan P) {
     extern __shared__ float sm[];
     __shared__ int listed;
     __shared__ Control2D c;
@@ -471,7 +474,6 @@ __global__ void __launch_bounds__(kResidentThreads, 1) residentRun(Grid2D g, Fie
             f.sxx1[k] = t[0]; f.sxx2[k] = t[1]; f.szz1[k] = t[2]; f.szz2[k] = t[3]; f.sxz1[k] = t[4]; f.sxz2[k] = t[5];
         }
     }
-    if (blockIdx.x == 0 && tid == 0) ctl->base = c.base + count;
 }
 
 }  // namespace seis2d
