@@ -185,6 +185,7 @@ struct seis2d_session {
     int runMode = kRunByRule;
     int64_t longSteps = 0;          // steps of the runs by rule that a persistent run would suit
     bool persistentPending = false; // a persistent run has not been checked yet
+    bool persistentCaptured = false; // one was captured: the caller's replays of it are not seen here
     BarrierLimits barrier{kBarrierCycles, -1};   // seis2d_debug_barrier_wait
     uint64_t launches = 0;
 
@@ -225,12 +226,14 @@ struct seis2d_session {
     }
     void sync() {
         GridSync state{};
-        const bool check = persistentPending;
+        const bool check = persistentPending || persistentCaptured;
         if (check) cudaCheck(cudaMemcpyAsync(&state, gridSync, sizeof(state), cudaMemcpyDeviceToHost, stream), "read run status");
         cudaCheck(cudaStreamSynchronize(stream), "cudaStreamSynchronize");
         if (check) {
             persistentPending = false;
-            if (state.failed) throw RuntimeError("A persistent run gave up at a grid barrier; its results are invalid");
+            if (!state.failed) return;
+            cudaCheck(cudaMemsetAsync(&gridSync->failed, 0, sizeof(gridSync->failed), stream), "clear run status");
+            throw RuntimeError("A persistent run gave up at a grid barrier; its results are invalid");
         }
     }
     ~seis2d_session() {
@@ -391,6 +394,9 @@ void launchPersistent(seis2d_session* s, int count) {
     });
     s->launches += 1;
     s->persistentPending = true;
+    cudaStreamCaptureStatus capturing = cudaStreamCaptureStatusNone;
+    cudaCheck(cudaStreamIsCapturing(s->stream, &capturing), "capture status");
+    s->persistentCaptured |= capturing != cudaStreamCaptureStatusNone;
 }
 
 cudaGraphExec_t batchGraph(seis2d_session* s, int batch, bool multi) {

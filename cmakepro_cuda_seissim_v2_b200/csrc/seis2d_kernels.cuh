@@ -782,17 +782,19 @@ __global__ void injectSources(Grid2D g, Fields2D f, const Control2D* __restrict_
 
 // State of the persistent runs (seis2d_resident.cuh).
 struct GridSync {
-    unsigned failed;    // a wait of the last run gave up; its results are invalid
+    unsigned failed;    // a wait of a run gave up and no synchronising call has said so yet
     unsigned first;     // number of the exchange before the run's first
     unsigned last;      // number of the run's last exchange
     unsigned pad;
 };
 
 // Prepares the steps that follow in the stream.  A persistent run's exchanges are numbered here
-// and not by the host, so that a replay of a captured run has numbers of its own too.
+// and not by the host, so that a replay of a captured run has numbers of its own too.  The failure of an
+// earlier run stays until the host has read it: cleared here, a run enqueued before the next
+// synchronising call would hide it and go on from the broken state.
 __global__ void configureRun(Control2D* ctl, Control2D value, GridSync* gs, unsigned exchanges) {
     *ctl = value;
-    if (exchanges) *gs = GridSync{0, gs->last, gs->last + exchanges, 0};
+    if (exchanges) *gs = GridSync{gs->failed, gs->last, gs->last + exchanges, 0};
 }
 
 // Completes the last step of a batch: its stress-type point source and its receivers, then

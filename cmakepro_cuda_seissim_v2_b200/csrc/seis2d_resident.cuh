@@ -20,7 +20,8 @@
 // 6.4 to 21 us.
 //
 // All waits are bounded (BarrierLimits): a CTA that gives up sets the failure flag, which the
-// others see in their own waits, and every CTA leaves the run.
+// others see in their own waits, and every CTA leaves the run.  The flag stands until a
+// synchronising call has reported it, and runs that find it set do nothing.
 #pragma once
 
 #include "seis2d_kernels.cuh"
@@ -224,6 +225,7 @@ __global__ void __launch_bounds__(kResidentThreads, 1) residentRun(Grid2D g, Fie
                                                                    int count, BarrierLimits lim, ResidentPlan P) {
     extern __shared__ float sm[];
     __shared__ int listed;
+    __shared__ unsigned failed;
     __shared__ Control2D c;
     const Tile<S> T(g, P, sm);
     int2* list = reinterpret_cast<int2*>(sm + residentArrays<S> * kArea);   // {receiver, cell} of the tile's receivers
@@ -231,6 +233,7 @@ __global__ void __launch_bounds__(kResidentThreads, 1) residentRun(Grid2D g, Fie
     if (tid == 0) {
         listed = 0;
         c = *ctl;
+        failed = *reinterpret_cast<volatile unsigned*>(&gs->failed);
     }
 
     // Every array with its halo.
@@ -288,7 +291,8 @@ __global__ void __launch_bounds__(kResidentThreads, 1) residentRun(Grid2D g, Fie
     }
     HaloWords<S> halo;
     halo.init(T);
-    __syncthreads();   // `listed` is 0, `c` is there
+    __syncthreads();   // `listed` is 0, `c` and `failed` are there
+    if (failed) return;   // an earlier run left the state half way, or this one has already
     if (c.gatherOn)
         for (int r = tid; r < c.rcvCount; r += blockDim.x) {
             const int k = c.rcvIdx[r], i = k / g.NX - T.top, jr = k % g.NX - T.left;
