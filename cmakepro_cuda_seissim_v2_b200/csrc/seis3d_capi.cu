@@ -1521,7 +1521,8 @@ int seis3d_extract_views(seis3d_session* s, const seis3d_context* c, float* outp
         if (std::memcmp(&expected, layout, sizeof(expected)) != 0)
             throw InvalidArgument("Seis3D: the view layout does not describe this session (use seis3d_make_view_layout).");
         const uint64_t count = volume ? layout->totalSamples3D : layout->volumeOffset3D;
-        if (!deviceRange(s, output, std::size_t(count) * 2 * sizeof(float)))
+        if (reinterpret_cast<uintptr_t>(output) % sizeof(float) != 0 ||
+            !deviceRange(s, output, std::size_t(count) * 2 * sizeof(float)))
             throw InvalidArgument("Seis3D: the view output must be a device buffer of 2 floats per sample.");
         if (!s->viewStats) cudaCheck(deviceMalloc(&s->viewStats, 8 * sizeof(unsigned)), "allocate view statistics");
         const unsigned initial[5] = {0u, 0u, 0x7f7fffffu, 0u, 0u};

@@ -117,6 +117,7 @@ __global__ void __launch_bounds__(kViewThreads) extractViews(const __grid_consta
     const unsigned slice1 = unsigned(L.sliceOffset3D[1]), slice2 = unsigned(L.sliceOffset3D[2]);
     const unsigned volume = unsigned(L.volumeOffset3D);
     const unsigned VX = L.volumeX3D, VY = L.volumeY3D;
+    const bool paired = reinterpret_cast<uintptr_t>(a.out) % 8 == 0;   // the output may start at any float
     ViewExtremes e{0.0f, 0.0f, 3.402823466e38f, 0.0f};
     bool bad = false;
     for (unsigned i = blockIdx.x * kViewThreads + threadIdx.x; i < limit; i += gridDim.x * kViewThreads) {
@@ -142,7 +143,13 @@ __global__ void __launch_bounds__(kViewThreads) extractViews(const __grid_consta
             s = viewResample<kWave, kMaterial>(a, fx, fy, fz);
         }
         const bool waveFinite = isfinite(s.value), materialFinite = isfinite(s.material), speedFinite = isfinite(s.magnitude);
-        reinterpret_cast<float2*>(a.out)[i] = make_float2(waveFinite ? s.value : 0, materialFinite ? s.material : 0);
+        const float wave = waveFinite ? s.value : 0, material = materialFinite ? s.material : 0;
+        if (paired) {
+            reinterpret_cast<float2*>(a.out)[i] = make_float2(wave, material);
+        } else {
+            a.out[2 * i] = wave;
+            a.out[2 * i + 1] = material;
+        }
         bad |= !waveFinite || !materialFinite || !speedFinite || s.material < 0;
         const bool physical = x >= 0 && x < a.nx && y >= 0 && y < a.ny && z >= 0 && z < a.nz;
         if ((physical || a.includeBoundary) && waveFinite) e.wave = fmaxf(e.wave, fabsf(s.value));
