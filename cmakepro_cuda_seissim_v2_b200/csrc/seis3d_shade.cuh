@@ -36,14 +36,16 @@ __host__ __device__ __forceinline__ float smoothstepf(float e0, float e1, float 
 }
 
 // Division by a number that many quotients share: its reciprocal once, then per quotient the
-// product and Markstein's residual correction, which rounds as the IEEE division does (the
-// operands here are far from overflow and underflow).
+// product and Markstein's residual correction, which rounds as the IEEE division does while
+// neither the quotient nor the residual leaves the normal range.  The quotient may: a diverging
+// wave over a small display scale overflows, and the residual of an infinite quotient is not a
+// number.  The product is the result then, infinite with the quotient's sign as the division's is.
 struct Divisor {
     float d, r;
     __device__ __forceinline__ explicit Divisor(float v) : d(v), r(1.0f / v) {}
     __device__ __forceinline__ float under(float x) const {
-        const float q = __fmul_rn(x, r);
-        return __fmaf_rn(__fmaf_rn(-d, q, x), r, q);
+        const float q = __fmul_rn(x, r), corrected = __fmaf_rn(__fmaf_rn(-d, q, x), r, q);
+        return fabsf(q) <= 3.402823466e38f ? corrected : q;
     }
 };
 
