@@ -248,8 +248,13 @@ struct seis2d_session {
 namespace {
 
 // One strip per block, and for the stresses a row of blocks that samples the receivers.
-dim3 stressGrid(const Grid2D& g, int scheme, int rows) { return dim3(stripsAcross(g), stressStrips(g, scheme, rows) + 1); }
-dim3 velocityGrid(const Grid2D& g, int rows) { return dim3(stripsAcross(g), velocityStrips(g, rows)); }
+dim3 stripGrid(const Grid2D& g, int down) {
+    constexpr int kMostY = 65535;
+    const int layers = (down + kMostY - 1) / kMostY;   // stripRow
+    return dim3(stripsAcross(g), (down + layers - 1) / layers, layers);
+}
+dim3 stressGrid(const Grid2D& g, int scheme, int rows) { return stripGrid(g, stressStrips(g, scheme, rows) + 1); }
+dim3 velocityGrid(const Grid2D& g, int rows) { return stripGrid(g, velocityStrips(g, rows)); }
 constexpr int kSourceThreads = 256;
 constexpr int kGraphBatch = 64;
 static_assert(kSourceThreads >= SEIS2D_MAX_ACTIVE_SOURCES, "one thread per active source");

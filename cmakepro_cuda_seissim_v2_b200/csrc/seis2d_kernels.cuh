@@ -338,6 +338,18 @@ __device__ __forceinline__ bool stressSource(const Control2D& c, int step, float
     return isfinite(w);
 }
 
+// ---- launch shapes -------------------------------------------------------------------------
+
+// Strips of a grid: across, and down for the stresses and the velocities.
+__host__ __device__ __forceinline__ int stripsAcross(const Grid2D& g) { return (g.NX - 8 + kCols - 1) / kCols; }
+__host__ __device__ __forceinline__ int stressStrips(const Grid2D& g, int scheme, int rows) {
+    return (g.NZ - 4 - (scheme == kFree ? g.fs : 4) + rows - 1) / rows;
+}
+__host__ __device__ __forceinline__ int velocityStrips(const Grid2D& g, int rows) { return (g.NZ - 8 + rows - 1) / rows; }
+// Place of a block among the strips down the grid.  They are numbered along y and go on along z: a
+// grid of a few columns can have more strips than the 65,535 blocks that y takes.
+__device__ __forceinline__ int stripRow() { return int(blockIdx.z * gridDim.y + blockIdx.y); }
+
 // ---- stress ----------------------------------------------------------------------------
 
 // Whether a strip of R rows has cells in the hybrid scheme's layer.  Strips without them run a body
@@ -513,13 +525,14 @@ __global__ void __launch_bounds__(kThreads) stressStep(Grid2D g, Fields2D f, con
     __shared__ Shared sh[kSharedArrays<S> * R];
     waitForPrevious();
     const Control2D c = *ctl;
-    const int step = c.base + slot;
-    if (blockIdx.y == gridDim.y - 1) {
+    const int step = c.base + slot, row = stripRow(), strips = stressStrips(g, S, R);
+    if (row >= strips) {
         // Receiver row: the velocities of step-1 are final while the stresses update.
-        if (slot > 0) recordStep<S>(g, f, c, step - 1, blockIdx.x * kThreads + threadIdx.x, kThreads * gridDim.x);
+        if (row == strips && slot > 0)
+            recordStep<S>(g, f, c, step - 1, blockIdx.x * kThreads + threadIdx.x, kThreads * gridDim.x);
         return;
     }
-    stressStrip<S, R>(g, f, c, step, slot > 0, blockIdx.x, blockIdx.y, sh);
+    stressStrip<S, R>(g, f, c, step, slot > 0, blockIdx.x, row, sh);
     launchDependents();
 }
 
@@ -709,8 +722,10 @@ template <int S, int R>
 __global__ void __launch_bounds__(kThreads) velocityStep(Grid2D g, Fields2D f, const Control2D* __restrict__ ctl, int slot) {
     __shared__ Shared sh[kSharedArrays<S> * R];
     waitForPrevious();
+    const int row = stripRow(), strips = velocityStrips(g, R);
+    if (row >= strips) return;
     const Control2D c = *ctl;
-    velocityStrip<S, R>(g, f, c, c.base + slot, blockIdx.x, blockIdx.y, blockIdx.y == gridDim.y - 1, sh);
+    velocityStrip<S, R>(g, f, c, c.base + slot, blockIdx.x, row, row == strips - 1, sh);
     launchDependents();
 }
 
@@ -837,15 +852,6 @@ struct BarrierLimits {
     long long cycles;     // bound of every wait
     int withheldBlock;    // test hook: this block sends nothing in its first exchange; -1 in use
 };
-
-// ---- launch shapes -------------------------------------------------------------------------
-
-// Strips of a grid: across, and down for the stresses and the velocities.
-__host__ __device__ __forceinline__ int stripsAcross(const Grid2D& g) { return (g.NX - 8 + kCols - 1) / kCols; }
-__host__ __device__ __forceinline__ int stressStrips(const Grid2D& g, int scheme, int rows) {
-    return (g.NZ - 4 - (scheme == kFree ? g.fs : 4) + rows - 1) / rows;
-}
-__host__ __device__ __forceinline__ int velocityStrips(const Grid2D& g, int rows) { return (g.NZ - 8 + rows - 1) / rows; }
 
 // recordReceiverStepOnGpu / copyReceiverRecordsFromGpu sample (Cuda_Check.cu:793-818).
 template <int S>
