@@ -187,6 +187,7 @@ struct seis2d_session {
     bool persistentPending = false; // a persistent run has not been checked yet
     bool persistentCaptured = false; // one was captured: the caller's replays of it are not seen here
     BarrierLimits barrier{kBarrierCycles, -1};   // seis2d_debug_barrier_wait
+    bool refusePersistent = false;               // seis2d_debug_refuse_persistent
     uint64_t launches = 0;
 
     template <class T> T* alloc(std::size_t count) {
@@ -387,21 +388,31 @@ bool residentReady(seis2d_session* s) {
     return true;
 }
 
-// One cooperative launch of `count` steps (after configure()).
-void launchPersistent(seis2d_session* s, int count) {
+// One cooperative launch of `count` steps (after configure()); false when it is refused, and then for all
+// later runs of the session.  The plan counts the device's SMs, and a context may have fewer (an
+// MPS share, a partition of the SMs): the steps are replayed there, as on grids that do not fit.
+bool launchPersistent(seis2d_session* s, int count) {
+    cudaError_t launched = cudaSuccess;
     dispatchResident(s, [&](auto tag, auto rows) {
         constexpr int S = decltype(tag)::value, R = decltype(rows)::value;
         void* args[] = {&s->g, &s->f, &s->ctl, &s->gridSync, &count, &s->barrier, &s->resident};
-        cudaCheck(cudaLaunchCooperativeKernel(reinterpret_cast<void*>(residentRun<S, R>),
-                                              dim3(s->resident.px * s->resident.pz), dim3(s->residentThreads), args,
-                                              s->residentShared, s->stream),
-                  "persistent launch");
+        launched = s->refusePersistent
+                       ? cudaErrorCooperativeLaunchTooLarge
+                       : cudaLaunchCooperativeKernel(reinterpret_cast<void*>(residentRun<S, R>),
+                                                     dim3(s->resident.px * s->resident.pz), dim3(s->residentThreads), args,
+                                                     s->residentShared, s->stream);
     });
+    if (launched != cudaSuccess) {
+        cudaGetLastError();
+        s->resident.px = 0;
+        return false;
+    }
     s->launches += 1;
     s->persistentPending = true;
     cudaStreamCaptureStatus capturing = cudaStreamCaptureStatusNone;
     cudaCheck(cudaStreamIsCapturing(s->stream, &capturing), "capture status");
     s->persistentCaptured |= capturing != cudaStreamCaptureStatusNone;
+    return true;
 }
 
 cudaGraphExec_t batchGraph(seis2d_session* s, int batch, bool multi) {
@@ -870,8 +881,7 @@ int seis2d_run_steps(seis2d_session* session, int first_it, int count, const sei
                                 residentReady(s);
         configure(s, runControl(s, *context, first_it, num_active_sources, num_active_sources >= 0),
                   persistent ? 2u * unsigned(count) : 0u);
-        if (persistent) {
-            launchPersistent(s, count);
+        if (persistent && launchPersistent(s, count)) {
             noteGather(s, first_it, count);
             return;
         }
@@ -1080,6 +1090,10 @@ int seis2d_debug_barrier_wait(seis2d_session* session, long long cycles, int wit
         s->barrier.cycles = cycles ? cycles : kBarrierCycles;
         s->barrier.withheldBlock = withheld_block;
     });
+}
+
+int seis2d_debug_refuse_persistent(seis2d_session* session, int refuse) {
+    return guarded([&] { checkedSession(session)->refusePersistent = refuse != 0; });
 }
 
 int seis2d_synchronize(seis2d_session* session) {

@@ -222,6 +222,9 @@ void seis2d_debug_fail_allocation(int nth);
  * synchronising call fails with SEIS2D_RUNTIME_ERROR.  -1 withholds nothing.  Meant for tests
  * of the failure path only. */
 int seis2d_debug_barrier_wait(seis2d_session* session, long long cycles, int withheld_block);
+/* Test hook (host-side fault injection): with refuse != 0 the session's cooperative launches are
+ * refused as a context with too few SMs refuses them; the steps are then replayed from graphs. */
+int seis2d_debug_refuse_persistent(seis2d_session* session, int refuse);
 /* Runs the session's later work on `stream` (a cudaStream_t; NULL = the legacy default
  * stream, where the reference enqueues its 2-D kernels, so plain cudaMemcpy calls of the
  * caller are ordered after the steps as they are with the reference).  The session's own
