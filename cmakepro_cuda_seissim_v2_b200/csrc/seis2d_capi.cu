@@ -363,6 +363,16 @@ bool residentPays(seis2d_session* s, int count) {
     return s->resident.mail || s->longSteps >= kResidentInvestment;
 }
 
+// While it lives, this thread may allocate although a capture of another stream is under way (that
+// capture would otherwise be ended with an error by the allocation).
+struct RelaxedCapture {
+    cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
+    RelaxedCapture() { cudaThreadExchangeStreamCaptureMode(&mode); }
+    ~RelaxedCapture() { cudaThreadExchangeStreamCaptureMode(&mode); }
+    RelaxedCapture(const RelaxedCapture&) = delete;
+    RelaxedCapture& operator=(const RelaxedCapture&) = delete;
+};
+
 // The mailboxes of persistent runs, from the first one on: at initialisation a session without
 // long runs would pay for them (on a small grid they are most of its memory).  Where they cannot
 // be had, or not now (the stream is being captured), the steps are replayed from graphs.
@@ -373,6 +383,8 @@ bool residentReady(seis2d_session* s) {
         cudaGetLastError();
         return false;
     }
+    // Callers step sessions during captures of other streams, and replayed steps do not allocate.
+    const RelaxedCapture relaxed;
     try {
         dispatchResident(s, [&](auto tag, auto rows) {
             cudaCheck(cudaFuncSetAttribute(residentRun<decltype(tag)::value, decltype(rows)::value>,
