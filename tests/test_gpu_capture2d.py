@@ -30,7 +30,6 @@ def test_stepping_during_another_capture(solver2d_lib, cuda_device):
                 y = x * 2.0
                 for n in range(BEFORE, RUNS):
                     seis2d.runGpuSimulationSteps(gpu, n * RUN, RUN, c)
-                    seis2d.synchronize(gpu)
                 y = y + 1.0
             graph.replay()
             torch.cuda.synchronize()
