@@ -229,13 +229,13 @@ struct seis3d_session {
     int device = 0;
     cudaStream_t stream = nullptr;
     int64_t pitch = 0, plane = 0;
-    float* pool = nullptr;          // kLead elements, then 12 padded volumes: 9 fields, 3 materials
+    float* pool = nullptr;          // the lead (kLead), then 12 padded volumes: 9 fields, 3 materials
     std::size_t poolBytes = 0;
     float* field[9]{};
     float* invRho = nullptr;
     float* lambda = nullptr;
     float* mu = nullptr;
-    float* psiPool[3]{};            // kLead elements, then the CPML memories
+    float* psiPool[3]{};            // the lead, then the CPML memories
     float* psi[3]{};                // CPML memories (FP32, or BF16 elements in SEIS3D_STORAGE_BF16_CPML)
     std::size_t psiCount[3]{};
     int storage = SEIS3D_STORAGE_FP32;
@@ -911,13 +911,15 @@ int seis3d_initialize(seis3d_session** out, const seis3d_context* context, const
             s->pitch = opt.compact_rows ? c.gx3D : roundUp(c.gx3D, 32);
             s->plane = s->pitch * c.gy3D;
             const std::size_t volume = std::size_t(s->plane) * c.gz3D;
-            s->poolBytes = (kLead + volume * 12) * sizeof(float);
+            // Unpitched rows start anywhere on a line, so their callers keep the allocation's own alignment.
+            const std::size_t lead = opt.compact_rows ? 0 : kLead;
+            s->poolBytes = (lead + volume * 12) * sizeof(float);
             cudaCheck(deviceMalloc(&s->pool, s->poolBytes), "allocate fields");
             cudaCheck(cudaMemsetAsync(s->pool, 0, s->poolBytes, s->stream), "clear fields");
-            for (int k = 0; k < 9; ++k) s->field[k] = s->pool + kLead + k * volume;
-            s->invRho = s->pool + kLead + 9 * volume;
-            s->lambda = s->pool + kLead + 10 * volume;
-            s->mu = s->pool + kLead + 11 * volume;
+            for (int k = 0; k < 9; ++k) s->field[k] = s->pool + lead + k * volume;
+            s->invRho = s->pool + lead + 9 * volume;
+            s->lambda = s->pool + lead + 10 * volume;
+            s->mu = s->pool + lead + 11 * volume;
             s->allocated = s->poolBytes;
             if (!c.reflecting3D) {
                 const int thick[3] = {2 * c.pml3D, 2 * c.pml3D, (c.freeSurface3D ? 1 : 2) * c.pml3D};
@@ -926,9 +928,9 @@ int seis3d_initialize(seis3d_session** out, const seis3d_context* context, const
                 s->psiCount[2] = std::size_t(6) * thick[2] * c.gy3D * s->pitch;
                 for (int a = 0; a < 3; ++a) {
                     // The x slab's rows are not x-pitched: its memories start at the allocation.
-                    const std::size_t lead = a == 0 ? 0 : kLead * s->memoryBytes();
-                    cudaCheck(deviceMalloc(&s->psiPool[a], lead + s->psiBytes(a)), "allocate CPML memories");
-                    s->psi[a] = s->psiPool[a] + lead / sizeof(float);
+                    const std::size_t leadBytes = a == 0 ? 0 : lead * s->memoryBytes();
+                    cudaCheck(deviceMalloc(&s->psiPool[a], leadBytes + s->psiBytes(a)), "allocate CPML memories");
+                    s->psi[a] = s->psiPool[a] + leadBytes / sizeof(float);
                     cudaCheck(cudaMemsetAsync(s->psi[a], 0, s->psiBytes(a), s->stream), "clear CPML");
                     s->allocated += s->psiBytes(a);
                     const auto k = coefficients(c, a);

@@ -30,7 +30,8 @@ constexpr int kRadius = 4;
 // interior cell of a pitched row (x = 4) starts a 128-byte line.  The 32-cell rows that the
 // passes stage, write and read memories of then cover 4 sectors of 32 bytes instead of 5, and
 // no sector is written by two CTAs (a halo row takes 6 instead of 5).  The same passes without
-// it: 300x300x400 1.354 ms a step against 1.260, 300x50x300 0.355 against 0.337.
+// it: 300x300x400 1.354 ms a step against 1.260, 300x50x300 0.355 against 0.337.  Sessions with
+// unpitched rows (compact_rows) have none.
 constexpr int kLead = 28;
 
 // Geometry shared by every kernel of a session.

@@ -138,7 +138,9 @@ typedef struct seis3d_options {
 
 /* Device views of a session (the GPUSimData3D members of include/Common3D.h:76-93).
  * Fields and materials use the padded X-contiguous layout of the reference with a row
- * pitch rounded up to 32 elements:  index(x,y,z) = (z*gy + y)*pitch + x.  In FP16/BF16
+ * pitch rounded up to 32 elements:  index(x,y,z) = (z*gy + y)*pitch + x.  The first updated cell
+ * of a row (x = 4) starts a 128-byte line and element 0 is 16-byte aligned; with compact_rows
+ * the pitch is gx3D and the first field starts an allocation (256 bytes).  In FP16/BF16
  * storage the pointers address 2-byte elements and field_scale[] holds the per-field
  * scale (stored = physical / scale). */
 typedef struct seis3d_device_views {
