@@ -268,7 +268,7 @@ template <class K> void launchStep(K kernel, dim3 grid, seis2d_session* s, int s
     attr.val.programmaticStreamSerializationAllowed = 1;
     cudaLaunchConfig_t cfg{};
     cfg.gridDim = grid;
-    cfg.blockDim = dim3(kThreads);
+    cfg.blockDim = dim3(stripThreads(s->g));
     cfg.stream = s->stream;
     cfg.attrs = &attr;
     cfg.numAttrs = overlap ? 1 : 0;

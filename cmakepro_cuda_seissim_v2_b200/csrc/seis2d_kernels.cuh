@@ -342,6 +342,11 @@ __device__ __forceinline__ bool stressSource(const Control2D& c, int step, float
 
 // Strips of a grid: across, and down for the stresses and the velocities.
 __host__ __device__ __forceinline__ int stripsAcross(const Grid2D& g) { return (g.NX - 8 + kCols - 1) / kCols; }
+// Threads of a strip's block: a grid narrower than one strip has no columns for the last warps, whose
+// registers would only keep other strips off the SM.  us per step with 128 threads and with these: 12x60000
+// split 94.6 / 45.9, 12x200000 hybrid 273.8 / 115.2, 40x50000 split 118.1 / 80.9 and with a free surface
+// 123.0 / 83.9, 60x20000 hybrid 43.9 / 33.5.
+inline int stripThreads(const Grid2D& g) { return g.NX < kThreads ? (g.NX + 31) / 32 * 32 : kThreads; }
 __host__ __device__ __forceinline__ int stressStrips(const Grid2D& g, int scheme, int rows) {
     return (g.NZ - 4 - (scheme == kFree ? g.fs : 4) + rows - 1) / rows;
 }
@@ -529,7 +534,7 @@ __global__ void __launch_bounds__(kThreads) stressStep(Grid2D g, Fields2D f, con
     if (row >= strips) {
         // Receiver row: the velocities of step-1 are final while the stresses update.
         if (row == strips && slot > 0)
-            recordStep<S>(g, f, c, step - 1, blockIdx.x * kThreads + threadIdx.x, kThreads * gridDim.x);
+            recordStep<S>(g, f, c, step - 1, blockIdx.x * blockDim.x + threadIdx.x, blockDim.x * gridDim.x);
         return;
     }
     stressStrip<S, R>(g, f, c, step, slot > 0, blockIdx.x, row, sh);
