@@ -16,6 +16,7 @@
 #include <cstring>
 #include <limits>
 #include <map>
+#include <mutex>
 #include <stdexcept>
 #include <string>
 #include <type_traits>
@@ -149,8 +150,29 @@ int kernelScheme(int flag, bool upFlag) {
 // (seis2d_resident.cuh).  But it also loads and stores the state and ends with a look at its status.  One run and a synchronise,
 // graph against persistent in us: 8 steps 123/134 (440x420, free surface), 105/100 (hybrid),
 // 77/76 (120x100, split); 16 steps 198/194, 170/156, 113/101; 2 steps 65/77, 62/72, 54/68.
+//
+// A persistent run has the chip to itself, replayed runs of several sessions share it.  So the rule also wants
+// that no other session's run is still going on the device (othersRunning).  us per step of one of 1 / 2 / 4 / 8
+// sessions with runs queued: 120x100 free surface all persistent 3.2 / 3.3 / 3.3 / 3.3, all replayed
+// 4.0 / 2.2 / 1.2 / 0.7, by rule 3.2 / 2.3 / 1.3 / 0.7; 250x300 hybrid 4.1 / 4.1 / 4.0 / 4.0, 5.5 / 3.4 / 2.1 / 2.1,
+// 4.1 / 3.5 / 2.2 / 2.1.
 constexpr int kRunByRule = -1;
 constexpr int kResidentSteps = 16, kResidentInvestment = 512;
+
+namespace {
+
+// The living sessions, so that they can see each other's runs (othersRunning).
+struct Sessions {
+    std::mutex mutex;
+    std::vector<seis2d_session*> all;
+    std::atomic<int> count{0};
+};
+Sessions& sessions() {
+    static Sessions* const s = new Sessions;   // a session may be released after static objects are
+    return *s;
+}
+
+}  // namespace
 
 struct seis2d_session {
     Grid2D g{};
@@ -177,6 +199,9 @@ struct seis2d_session {
     float* gatherVz = nullptr;
     int gatherReceivers = 0, gatherStart = 0, gatherStride = 1, gatherSamples = 0, gatherTaken = 0;
     bool gatherOn = false;
+    int device = 0;
+    cudaEvent_t ran = nullptr;             // the end of the session's last run of many steps
+    std::atomic<bool> hasRun{false};       // `ran` has been recorded
     std::map<std::pair<int, int>, cudaGraphExec_t> graphs;  // (batch, with multi-source) -> graph
     GridSync* gridSync = nullptr;   // failure state of the persistent runs
     ResidentPlan resident{};        // tiles of the persistent runs (px = 0: the grid does not fit on the chip)
@@ -237,7 +262,19 @@ struct seis2d_session {
             throw RuntimeError("A persistent run gave up at a grid barrier; its results are invalid");
         }
     }
+    seis2d_session() {
+        const std::lock_guard<std::mutex> lock(sessions().mutex);
+        sessions().all.push_back(this);
+        ++sessions().count;
+    }
     ~seis2d_session() {
+        {
+            const std::lock_guard<std::mutex> lock(sessions().mutex);
+            auto& all = sessions().all;
+            all.erase(std::find(all.begin(), all.end(), this));
+            --sessions().count;
+        }
+        if (ran) cudaEventDestroy(ran);
         for (auto& kv : graphs) cudaGraphExecDestroy(kv.second);
         if (stream) cudaStreamSynchronize(stream);
         if (own && own != stream) cudaStreamSynchronize(own);
@@ -355,16 +392,8 @@ void planResident(seis2d_session* s, int sms, std::size_t sharedLimit) {
 
 std::size_t mailBytes(const ResidentPlan& p) { return std::size_t(p.px) * p.pz * 8 * p.side * sizeof(uint4); }
 
-// Whether a run of `count` steps by rule is persistent (kRunByRule).  The mailboxes are taken when the
-// session's long runs have come to kResidentInvestment steps: allocating them takes about 0.4 ms.
-bool residentPays(seis2d_session* s, int count) {
-    if (count < kResidentSteps || (s->scheme != kHybrid && s->residentRows > 2)) return false;
-    s->longSteps = std::min<int64_t>(s->longSteps + count, kResidentInvestment);
-    return s->resident.mail || s->longSteps >= kResidentInvestment;
-}
-
-// While it lives, this thread may allocate although a capture of another stream is under way (that
-// capture would otherwise be ended with an error by the allocation).
+// While it lives, this thread may allocate and look at events although a capture of another stream is under
+// way (which such a call would otherwise end with an error).
 struct RelaxedCapture {
     cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
     RelaxedCapture() { cudaThreadExchangeStreamCaptureMode(&mode); }
@@ -372,6 +401,39 @@ struct RelaxedCapture {
     RelaxedCapture(const RelaxedCapture&) = delete;
     RelaxedCapture& operator=(const RelaxedCapture&) = delete;
 };
+
+// Whether another session's last run is still going on the device.  This decides only how a run is launched:
+// the results are the same bits either way.
+bool othersRunning(const seis2d_session* s) {
+    const RelaxedCapture relaxed;
+    const std::lock_guard<std::mutex> lock(sessions().mutex);
+    for (const seis2d_session* o : sessions().all)
+        if (o != s && o->device == s->device && o->hasRun && cudaEventQuery(o->ran) == cudaErrorNotReady) {
+            cudaGetLastError();
+            return true;
+        }
+    return false;
+}
+
+// Marks the end of a run for the other sessions, if there are any (a microsecond of a call's 36); not in a
+// capture, whose replays are the caller's.
+void noteRun(seis2d_session* s) {
+    if (sessions().count < 2) return;
+    cudaStreamCaptureStatus capturing = cudaStreamCaptureStatusNone;
+    if (cudaStreamIsCapturing(s->stream, &capturing) == cudaSuccess && capturing == cudaStreamCaptureStatusNone &&
+        cudaEventRecord(s->ran, s->stream) == cudaSuccess)
+        s->hasRun = true;
+    else
+        cudaGetLastError();
+}
+
+// Whether a run of `count` steps by rule is persistent (kRunByRule).  The mailboxes are taken when the
+// session's long runs have come to kResidentInvestment steps: allocating them takes about 0.4 ms.
+bool residentPays(seis2d_session* s, int count) {
+    if (count < kResidentSteps || (s->scheme != kHybrid && s->residentRows > 2)) return false;
+    s->longSteps = std::min<int64_t>(s->longSteps + count, kResidentInvestment);
+    return (s->resident.mail || s->longSteps >= kResidentInvestment) && !othersRunning(s);
+}
 
 // The mailboxes of persistent runs, from the first one on: at initialisation a session without
 // long runs would pay for them (on a small grid they are most of its memory).  Where they cannot
@@ -788,6 +850,8 @@ int seis2d_initialize(seis2d_session** session, const seis2d_context* context) {
                 const std::size_t lines = 4 + (c.flag_type == 3 ? 1 : 0);
                 int cooperative = 0, device = 0, sms = 0, shared = 0;
                 cudaCheck(cudaGetDevice(&device), "device");
+                s->device = device;
+                cudaCheck(cudaEventCreateWithFlags(&s->ran, cudaEventDisableTiming), "run event");
                 cudaCheck(cudaDeviceGetAttribute(&cooperative, cudaDevAttrCooperativeLaunch, device), "cooperative launch");
                 cudaCheck(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device), "SM count");
                 cudaCheck(cudaDeviceGetAttribute(&shared, cudaDevAttrMaxSharedMemoryPerBlockOptin, device), "shared memory");
@@ -894,6 +958,7 @@ int seis2d_run_steps(seis2d_session* session, int first_it, int count, const sei
         configure(s, runControl(s, *context, first_it, num_active_sources, num_active_sources >= 0),
                   persistent ? 2u * unsigned(count) : 0u);
         if (persistent && launchPersistent(s, count)) {
+            noteRun(s);
             noteGather(s, first_it, count);
             return;
         }
@@ -904,6 +969,7 @@ int seis2d_run_steps(seis2d_session* session, int first_it, int count, const sei
             s->launches += uint64_t(batch) * (multi ? 3 : 2) + 1;
             done += batch;
         }
+        noteRun(s);
         noteGather(s, first_it, count);
     });
 }

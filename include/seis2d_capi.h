@@ -234,7 +234,7 @@ int seis2d_set_stream(seis2d_session* session, void* stream);
  * launch that keeps the state on the chip, or graph replay.  Until a mode is set the library
  * chooses: long runs (16 steps or more, once a session has made 512 of them) on grids that fit
  * on the chip (on a B200 up to 227,000 cells in the hybrid scheme, 151,000 in the others) are
- * persistent.  A grid of more than 227,000 cells is replayed in either mode.  The results are
+ * persistent while no other session's run is going on the device.  A grid of more than 227,000 cells is replayed in either mode.  The results are
  * the same bits. */
 enum seis2d_run_mode { SEIS2D_RUN_PERSISTENT = 0, SEIS2D_RUN_GRAPH = 1 };
 int seis2d_set_run_mode(seis2d_session* session, int mode);
