@@ -311,11 +311,14 @@ template <class K> void launchStep(K kernel, dim3 grid, seis2d_session* s, int s
     cfg.numAttrs = overlap ? 1 : 0;
     cudaCheck(cudaLaunchKernelEx(&cfg, kernel, s->g, s->f, static_cast<const Control2D*>(s->ctl), slot), "step kernel launch");
 }
+// The kernels with strips along z are those of the most rows: grids so tall are large (stripRows).
 template <int S, int R> void launchStress(seis2d_session* s, int slot, bool overlap) {
-    launchStep(stressStep<S, R>, stressGrid(s->g, S, R), s, slot, overlap);
+    const dim3 grid = stressGrid(s->g, S, R);
+    launchStep(R == 4 && grid.z > 1 ? stressStep<S, R, R == 4> : stressStep<S, R, false>, grid, s, slot, overlap);
 }
 template <int S, int R> void launchVelocity(seis2d_session* s, int slot, bool overlap) {
-    launchStep(velocityStep<S, R>, velocityGrid(s->g, R), s, slot, overlap);
+    const dim3 grid = velocityGrid(s->g, R);
+    launchStep(R == 4 && grid.z > 1 ? velocityStep<S, R, R == 4> : velocityStep<S, R, false>, grid, s, slot, overlap);
 }
 template <int S> void launchInject(seis2d_session* s) {
     injectSources<S><<<1, kSourceThreads, 0, s->stream>>>(s->g, s->f, s->ctl);

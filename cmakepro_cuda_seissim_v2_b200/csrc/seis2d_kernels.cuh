@@ -525,19 +525,23 @@ __device__ __forceinline__ void stressStrip(const Grid2D& g, const Fields2D& f, 
     }
 }
 
-template <int S, int R>
+// kTall: the strips go on along gridDim.z (stripRow).  Grids that do not need that have kernels without it: with
+// it in theirs, 1601x1203 cells in the hybrid scheme took 36.5 us a step instead of 35.8 and 250x300 5.9
+// instead of 5.7.
+template <int S, int R, bool kTall>
 __global__ void __launch_bounds__(kThreads) stressStep(Grid2D g, Fields2D f, const Control2D* __restrict__ ctl, int slot) {
     __shared__ Shared sh[kSharedArrays<S> * R];
     waitForPrevious();
     const Control2D c = *ctl;
-    const int step = c.base + slot, row = stripRow(), strips = stressStrips(g, S, R);
-    if (row >= strips) {
+    const int step = c.base + slot;
+    const bool receivers = kTall ? stripRow() >= stressStrips(g, S, R) : blockIdx.y == gridDim.y - 1;
+    if (receivers) {
         // Receiver row: the velocities of step-1 are final while the stresses update.
-        if (row == strips && slot > 0)
+        if (slot > 0 && (!kTall || stripRow() == stressStrips(g, S, R)))
             recordStep<S>(g, f, c, step - 1, blockIdx.x * blockDim.x + threadIdx.x, blockDim.x * gridDim.x);
         return;
     }
-    stressStrip<S, R>(g, f, c, step, slot > 0, blockIdx.x, row, sh);
+    stressStrip<S, R>(g, f, c, step, slot > 0, blockIdx.x, kTall ? stripRow() : blockIdx.y, sh);
     launchDependents();
 }
 
@@ -723,14 +727,14 @@ __device__ __forceinline__ void velocityStrip(const Grid2D& g, const Fields2D& f
     }
 }
 
-template <int S, int R>
+template <int S, int R, bool kTall>
 __global__ void __launch_bounds__(kThreads) velocityStep(Grid2D g, Fields2D f, const Control2D* __restrict__ ctl, int slot) {
     __shared__ Shared sh[kSharedArrays<S> * R];
     waitForPrevious();
-    const int row = stripRow(), strips = velocityStrips(g, R);
-    if (row >= strips) return;
+    if (kTall && stripRow() >= velocityStrips(g, R)) return;
     const Control2D c = *ctl;
-    velocityStrip<S, R>(g, f, c, c.base + slot, blockIdx.x, row, row == strips - 1, sh);
+    const bool last = kTall ? stripRow() == velocityStrips(g, R) - 1 : blockIdx.y == gridDim.y - 1;
+    velocityStrip<S, R>(g, f, c, c.base + slot, blockIdx.x, kTall ? stripRow() : blockIdx.y, last, sh);
     launchDependents();
 }
 
