@@ -37,15 +37,26 @@ __host__ __device__ __forceinline__ float smoothstepf(float e0, float e1, float 
 
 // Division by a number that many quotients share: its reciprocal once, then per quotient the
 // product and Markstein's residual correction, which rounds as the IEEE division does while
-// neither the quotient nor the residual leaves the normal range.  The quotient may: a diverging
-// wave over a small display scale overflows, and the residual of an infinite quotient is not a
-// number.  The product is the result then, infinite with the quotient's sign as the division's is.
+// neither the quotient nor the residual leaves the normal range (tests/test_gpu_division.py).
 struct Divisor {
     float d, r;
     __device__ __forceinline__ explicit Divisor(float v) : d(v), r(1.0f / v) {}
     __device__ __forceinline__ float under(float x) const {
-        const float q = __fmul_rn(x, r), corrected = __fmaf_rn(__fmaf_rn(-d, q, x), r, q);
-        return fabsf(q) <= 3.402823466e38f ? corrected : q;
+        const float q = __fmul_rn(x, r);
+        return __fmaf_rn(__fmaf_rn(-d, q, x), r, q);
+    }
+    // For quotients that may overflow: a diverging wave over a small display scale does.  The residual of an
+    // infinite quotient is not a number; the product is the result then, infinite with the quotient's sign
+    // as the division's is.  (For every quotient of a sample this cost 4 to 7 % of the kernel.)
+    __device__ __forceinline__ float underWide(float x) const {
+        const float q = __fmul_rn(x, r);
+        return fabsf(q) <= 3.402823466e38f ? __fmaf_rn(__fmaf_rn(-d, q, x), r, q) : q;
+    }
+    // The quotient clamped to [0, 1] (d > 0), from a product clamped before the correction: any x but a NaN then
+    // has a residual, and both clamps are part of their instructions.
+    __device__ __forceinline__ float fraction(float x) const {
+        const float q = __saturatef(__fmul_rn(x, r));
+        return __saturatef(__fmaf_rn(__fmaf_rn(-d, q, x), r, q));
     }
 };
 
@@ -117,7 +128,7 @@ __global__ void __launch_bounds__(256) shadeSlices(const float2* __restrict__ vi
 
 // The same two functions with the divisors that a ray's samples share.
 __device__ __forceinline__ float waveVisibility(const seis3d_transfer& t, const Divisor& span, float magnitude) {
-    const float visible = clampf(span.under(magnitude - t.waveThreshold3D), 0.0f, 1.0f);
+    const float visible = span.fraction(magnitude - t.waveThreshold3D);
     return powf(visible, fmaxf(t.waveGamma3D, 0.1f));
 }
 
@@ -253,7 +264,7 @@ __global__ void __launch_bounds__(32) renderVolume(VolumeTexture vol, const __gr
             if (done || i + k >= steps) break;
             const float2 sample = samples[k];
             const bool boundary = boundaries[k];
-            const float scalar = scaleFloor.under(sample.x * u.gain3D * u.volumeGain3D);
+            const float scalar = scaleFloor.underWide(sample.x * u.gain3D * u.volumeGain3D);
             const float magnitude = fabsf(scalar);
             const bool visible = !(t.displayMode3D == 2 || magnitude <= u.threshold3D);
             float waveDensity = 0.0f;
@@ -267,7 +278,7 @@ __global__ void __launch_bounds__(32) renderVolume(VolumeTexture vol, const __gr
             const float density = waveDensity + materialDensity;
             const float alpha = 1.0f - expf(-density * delta);
             const Rgb tint = boundary ? rgb(.78f, .53f, .20f)
-                                      : materialStop(t, ranged ? clampf(materialSpan.under(sample.y - materialLow), 0.0f, 1.0f) : 0.5f);
+                                      : materialStop(t, ranged ? materialSpan.fraction(sample.y - materialLow) : 0.5f);
             const Divisor norm(fmaxf(density, 1e-10f));
             // One rounding order whatever the compiler would fuse.
             auto blend = [&](float a, float b) { return __fmaf_rn(b, materialDensity, __fmul_rn(a, waveDensity)); };

@@ -20,8 +20,12 @@ __global__ void checkMeans(const float* a, const float* b, long long n, unsigned
 
 __global__ void checkQuotients(const float* x, const float* d, long long n, unsigned long long* wrong) {
     for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x) {
-        const float q = seis3d::shade::Divisor(d[i]).under(x[i]);
-        if (!same(q, __fdiv_rn(x[i], d[i]))) atomicAdd(wrong, 1ULL);
+        const seis3d::shade::Divisor by(d[i]);
+        const float exact = __fdiv_rn(x[i], d[i]);
+        // A quotient that overflows is not the plain form's case.
+        if (!same(by.underWide(x[i]), exact) || (isfinite(exact) && !same(by.under(x[i]), exact)) ||
+            !same(by.fraction(x[i]), fminf(fmaxf(exact, 0.0f), 1.0f)))
+            atomicAdd(wrong, 1ULL);
     }
 }
 

@@ -86,7 +86,7 @@ def test_buoyancy_means_of_hard_sums(check):
 # Numerators and divisors: ray positions over extents, wave values over the display scale, magnitudes over
 # the threshold's span, materials over their range, colours over densities.
 @pytest.mark.parametrize("x,d", [((1e-6, 4.0), (1e-3, 1.0)), ((1e-25, 1e10), (1e-20, 1e10)), ((1e-12, 1e6), (1e-6, 1.0)),
-                                 ((1e-3, 5e4), (1e-6, 5e4)), ((1e-20, 1e3), (1e-10, 1e3))])
+                                 ((1e-3, 5e4), (1e-6, 5e4)), ((1e-20, 1e3), (1e-10, 1e3)), ((0.999, 1.001), (0.999, 1.001))])
 def test_renderer_quotients(x, d, check):
     assert check(False, spread(*x, 4, signed=True), spread(*d, 5)) == 0
 
