@@ -259,7 +259,7 @@ struct seis2d_session {
             persistentPending = false;
             if (!state.failed) return;
             cudaCheck(cudaMemsetAsync(&gridSync->failed, 0, sizeof(gridSync->failed), stream), "clear run status");
-            throw RuntimeError("A persistent run gave up at a grid barrier; its results are invalid");
+            throw RuntimeError("A persistent run gave up at a grid barrier (a wait for a neighbouring tile's halo ran out); its results are invalid");
         }
     }
     seis2d_session() {
@@ -369,8 +369,9 @@ template <class F> void dispatchResident(const seis2d_session* s, F&& fn) {
 
 // Tiles of a persistent run: one per SM at most, fewest rows per thread first, then the shortest
 // halo.  A tile side is at least the halo, so that halos come from direct neighbours.  Three rows
-// per thread is where the split schemes' arrays fill an SM's shared memory: 512 threads, 148 SMs
-// and 227k cells at most (460x460).
+// per thread is where the split schemes' arrays fill an SM's shared memory.  So 148 SMs take at most
+// 148 x 512 cells a row of the threads, 227,000 with three, and which grids fit depends on their sides:
+// 465x465 does, 470x470 and 514x401 do not.
 void planResident(seis2d_session* s, int sms, std::size_t sharedLimit) {
     const Grid2D& g = s->g;
     const int words = s->scheme == kHybrid ? 1 : 2, arrays = s->scheme == kHybrid ? int(kHybridArrays) : int(kSplitArrays);

@@ -576,13 +576,11 @@ void launchPass(PassKernel kernel, const Shape& sh, std::size_t smem, cudaStream
     cudaCheck(cudaLaunchKernelEx(&launch.cfg, kernel, G, F, S, Q), what);
 }
 
-// Images of the velocities or the stresses at the free surface (in a step the passes write those
-// they read themselves).
-void launchSurfaceImages(seis3d_session* s, bool velocities, cudaStream_t stream) {
+// Images of the stresses at the free surface (in a step the passes write those they read themselves).
+void launchSurfaceImages(seis3d_session* s, cudaStream_t stream) {
     if (!s->ctx.freeSurface3D) return;
     const dim3 b(32, 8), g((s->ctx.gx3D - 8 + 31) / 32, (s->ctx.gy3D - 8 + 7) / 8);
-    if (velocities) velocityImages<<<g, b, 0, stream>>>(s->geometry(), s->fields());
-    else stressImages<<<g, b, 0, stream>>>(s->geometry(), s->fields());
+    stressImages<<<g, b, 0, stream>>>(s->geometry(), s->fields());
     launchCheck("free-surface images");
     ++s->launches;
 }
@@ -598,10 +596,11 @@ void launchWallImages(seis3d_session* s, bool velocities, cudaStream_t stream, b
     ++s->launches;
 }
 
-void launchImages(seis3d_session* s, bool velocities, cudaStream_t stream = nullptr) {
+// Both images of the stresses.
+void launchImages(seis3d_session* s, cudaStream_t stream = nullptr) {
     if (!stream) stream = s->stream;
-    launchSurfaceImages(s, velocities, stream);
-    launchWallImages(s, velocities, stream, false);
+    launchSurfaceImages(s, stream);
+    launchWallImages(s, false, stream, false);
 }
 
 // One leapfrog step in the reference order (cuda/Cuda_Seis3D.cu:602-624): the device clock's step
@@ -639,11 +638,11 @@ void enqueueStep(seis3d_session* s, const SourceParams& S, int slot, bool tail, 
     if (ev) cudaEventRecord(ev->afterStress, stream);
     launchWallImages(s, false, stream, !ev);
     if (s->net) {
-        launchSurfaceImages(s, false, stream);
+        launchSurfaceImages(s, stream);
         // Learned thin boundary: corrections of the boundary columns after the full step (on
         // the imaged state), then the stress images again for the corrected cells.
         enqueueBoundaryCorrection(s, stream);
-        launchImages(s, false, stream);
+        launchImages(s, stream);
     }
     if (tail) {
         stepTail<<<1, 256, 0, stream>>>(G, F, s->recv, s->recvCount, gather);
@@ -1023,7 +1022,7 @@ int seis3d_run_step(seis3d_session* s, const seis3d_context* c, const seis3d_sou
         requireSameGrid(s, c);
         adoptScalars(s, c);
         syncClock(s, step);
-        launchImages(s, false);
+        launchImages(s);
         enqueueSteps(s, sourceParams(s->ctx, *src), 1);
         closingImages(s);
         s->hostClock = step + 1;
@@ -1074,7 +1073,7 @@ int seis3d_run_steps(seis3d_session* s, const seis3d_context* c, const seis3d_so
         syncClock(s, first);
         const SourceParams S = sourceParams(s->ctx, *src);
         // Start-of-step stress images once; later steps inherit them from the step before.
-        launchImages(s, false);
+        launchImages(s);
         int done = 0;
         if (count >= kGraphBatch) {
             ensureGraph(s, *src, S);
@@ -1463,7 +1462,7 @@ int seis3d_profile_steps(seis3d_session* s, const seis3d_context* c, const seis3
         adoptScalars(s, c);
         syncClock(s, first);
         const SourceParams S = sourceParams(s->ctx, *src);
-        launchImages(s, false);
+        launchImages(s);
         std::vector<PassEvents> ev(static_cast<std::size_t>(count));
         for (auto& e : ev)
             for (cudaEvent_t* p : {&e.start, &e.afterVelocity, &e.afterImages, &e.afterStress, &e.end})
@@ -1538,7 +1537,6 @@ int seis3d_extract_views(seis3d_session* s, const seis3d_context* c, float* outp
         a.nx = s->ctx.nx3D; a.ny = s->ctx.ny3D; a.nz = s->ctx.nz3D;
         a.layout = *layout;
         a.sx = slices[0]; a.sy = slices[1]; a.sz = slices[2];
-        a.component = component; a.materialComponent = material_component;
         a.includeBoundary = include_boundary != 0;
         a.out = output;
         a.stats = s->viewStats;

@@ -6,8 +6,8 @@
 // colour statistics (largest |value|, material range, largest velocity magnitude).
 //
 // The per-sample arithmetic is the reference's (collocated face velocities, material
-// transforms, trilinear weights), read from this solver's pitched volumes.  One thread per
-// output sample; output samples are independent.
+// transforms, trilinear weights), read from this solver's pitched volumes.  Output samples are
+// independent; the grid strides over them.
 #pragma once
 
 #include "../../include/seis3d_capi.h"
@@ -27,7 +27,6 @@ struct ViewArgs {
     int nx, ny, nz;         // physical size
     seis3d_view_layout layout;
     int sx, sy, sz;
-    int component, materialComponent;
     int includeBoundary;
     float* out;
     unsigned* stats;        // [0] |value| max, [2] material min, [3] material max, [4] |v| max

@@ -231,11 +231,14 @@ int seis2d_debug_refuse_persistent(seis2d_session* session, int refuse);
  * non-blocking stream is the default; the previous stream is synchronised first. */
 int seis2d_set_stream(seis2d_session* session, void* stream);
 /* How seis2d_run_steps executes single-source runs (no reference counterpart): one cooperative
- * launch that keeps the state on the chip, or graph replay.  Until a mode is set the library
- * chooses: long runs (16 steps or more, once a session has made 512 of them) on grids that fit
- * on the chip (on a B200 up to 227,000 cells in the hybrid scheme, 151,000 in the others) are
- * persistent while no other session's run is going on the device.  A grid of more than 227,000 cells is replayed in either mode.  The results are
- * the same bits. */
+ * launch that keeps the state on the chip (persistent), or graph replay.  The results are the same bits.
+ * Until a mode is set the library chooses.  A run is persistent if it has 16 steps or more, the session
+ * has made 512 steps in such runs (the run that comes to them allocates a few MB), no other session's
+ * run is going on the device, and the grid fits on the chip.  On a B200 that is at most 151,000 cells
+ * (227,000 in the hybrid scheme), depending on the sides: 384x384 fits, 388x388 does not (hybrid: 468x468
+ * and 470x470).  With SEIS2D_RUN_PERSISTENT every run on a grid that fits is persistent, and what fits is the
+ * hybrid scheme's for all.  Runs with a gather of more than 1024 receivers, and all runs of a session
+ * whose cooperative launch was refused, are replayed in either mode. */
 enum seis2d_run_mode { SEIS2D_RUN_PERSISTENT = 0, SEIS2D_RUN_GRAPH = 1 };
 int seis2d_set_run_mode(seis2d_session* session, int mode);
 /* Device time of count steps replayed as in seis2d_run_steps, split into the stress and
