@@ -201,7 +201,8 @@ constexpr int kRaySamples = 4;   // samples of a ray whose texels are loaded tog
 // wave colour is left out where the wave has no density, a block is one warp of 8 x 4 pixels, and
 // the texels of four samples load together.  640 x 640: 460 us before, 345 with the first
 // two, 335 with one-warp blocks, 298 with four samples (two: 315); 1536 x 1536: 905 before,
-// 700 (660 with two samples at a time).  Same pixels.
+// 700 (660 with two samples at a time).  Same pixels.  Clamping the wave's visibility and the place in the material
+// range in their products (Divisor::fraction) took another view from 877 to 848 at 1536 x 1536.
 __global__ void __launch_bounds__(32) renderVolume(VolumeTexture vol, const __grid_constant__ seis3d_transfer t,
                                                     const __grid_constant__ seis3d_volume_view u, int width,
                                                     int height, int format, void* out) {
