@@ -130,6 +130,7 @@ class GPUSimData:
 
     def __init__(self):
         self._handle = c_void_p()
+        self._gather_receivers = 0   # of the last gather begun
 
     @property
     def handle(self) -> c_void_p:
@@ -326,11 +327,13 @@ def recordReceiverStepOnGpu(gpu: GPUSimData, num_rcv: int, out_vx: np.ndarray | 
 
 def gatherBegin(gpu: GPUSimData, capture_start_step: int, stride: int, samples: int) -> None:
     _check(_lib().seis2d_gather_begin(_session(gpu), int(capture_start_step), int(stride), int(samples)))
+    gpu._gather_receivers = int(gpu.views().receiverCapacity)
 
 
 def gatherFetch(gpu: GPUSimData, samples: int):
     """(vx, vz, taken): [receiver][sample] float32 traces and the samples recorded so far."""
-    n = max(gpu.views().receiverCapacity, 1)
+    # The gather keeps the receivers it began with, whatever receivers the session has since been given.
+    n = max(gpu.views().receiverCapacity, gpu._gather_receivers, 1)
     vx = np.zeros((n, samples), np.float32)
     vz = np.zeros((n, samples), np.float32)
     taken = c_int()
